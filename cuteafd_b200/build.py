@@ -23,13 +23,13 @@ LIB = OUT / "libcuteafd_b200.so"
 STAMP = OUT / "build" / "full.stamp"        # hash of the sources the full library was built from
 
 # what one family's single-GPU engine launches: enough for a checkout that only serves that family
-SUBSETS = {"latent_stack": (["runtime", "elementwise", "moe", "sampling", "tc_gemm", "attention_mla", "attention_mla_prefill", "latent_stack", "f32_linear"],
+SUBSETS = {"latent_stack": (["runtime", "elementwise", "moe", "sampling", "tc_gemm", "tc_gemm_wide", "attention_mla", "attention_mla_prefill", "latent_stack", "f32_linear"],
                             ["-DCA_TC_BF16_ONLY"]),
-           "hybrid_stack": (["runtime", "elementwise", "sampling", "tc_gemm", "attention_tc", "attention_mla_prefill", "hybrid_stack", "f32_linear"],
+           "hybrid_stack": (["runtime", "elementwise", "sampling", "tc_gemm", "tc_gemm_wide", "attention_tc", "attention_mla_prefill", "hybrid_stack", "f32_linear"],
                             ["-DCA_TC_BF16_ONLY"]),
-           "hyper_stack": (["runtime", "elementwise", "moe", "sampling", "tc_gemm", "attention_tc", "attention_mla_prefill", "hybrid_stack", "hyper_stack", "decay_scan", "f32_linear"],
+           "hyper_stack": (["runtime", "elementwise", "moe", "sampling", "tc_gemm", "tc_gemm_wide", "attention_tc", "attention_mla_prefill", "hybrid_stack", "hyper_stack", "decay_scan", "f32_linear"],
                            ["-DCA_TC_BF16_ONLY"]),
-           "mixed_stack": (["runtime", "elementwise", "sampling", "tc_gemm", "attention_tc", "attention_mla", "attention_mla_prefill", "hybrid_stack", "latent_stack", "hyper_stack", "decay_scan",
+           "mixed_stack": (["runtime", "elementwise", "sampling", "tc_gemm", "tc_gemm_wide", "attention_tc", "attention_mla", "attention_mla_prefill", "hybrid_stack", "latent_stack", "hyper_stack", "decay_scan",
                             "mixed_stack", "f32_linear"], ["-DCA_TC_BF16_ONLY"])}
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

@@ -23,7 +23,7 @@
 // (native/shared/cuda/linear.cu:865-1350).
 #define CA_PDL_CLASS 1
 #include <stdlib.h>
-#include "common.cuh"
+#include "tc_gemm_wide.cuh"
 
 // KIND_W4A8: MXFP4 weights (E2M1 + UE8M0 / 32, unpacked by TMA into 8-bit containers) x FP8 E4M3 activations with UE8M0 / 32
 // scales, kind::mxf8f6f4 (K = 32 per instruction) - the reference's default expert arithmetic
@@ -1062,6 +1062,20 @@ extern "C" int cuteafd_tc_linear(int kind, int swiglu, int tn, const void* tmA, 
       if (kind == KIND_NVFP4) return tn == 16 ? launch_cluster<KIND_NVFP4, 16>(a, grid_c, stream) : launch_cluster<KIND_NVFP4, 32>(a, grid_c, stream);
       return tn == 16 ? launch_cluster<KIND_MXFP4, 16>(a, grid_c, stream) : launch_cluster<KIND_MXFP4, 32>(a, grid_c, stream);
 #endif
+    }
+  }
+  // 128-row token tiles take the wide kernel where its units (128 tokens x 256 weight rows) occupy a quarter of the SMs: 4096 bf16 rows x 12288 x
+  // 2048 take 160 us there and 420 here, 300 NVFP4 rows x 9216 x 4096 18 and 36, 1024 bf16 rows x 2048 x 4096 (32 units) 26 and 31.  Below that
+  // the narrow kernel's split of K is the better use of the machine.
+  if (tn == 128 && max_ctas <= 0 && a.splits == 1 && kind != KIND_W4A8 && !peer.n && !grp_rows && act < 2 && !a.trace &&
+      (kind == KIND_BF16 || (ldsfb % 16 == 0 && ((uintptr_t)sfb & 15) == 0) || (kind == KIND_MXFP4 && ldsfb % 8 == 0 && ((uintptr_t)sfb & 7) == 0))) {
+    const long long items = tiles ? max_tiles : (rows_total + 127) / 128, units = items * (swiglu ? n_nt : (N + 255) / 256);
+    if (4 * units >= ca_sm_count()) {
+      WideArgs wa = {};
+      wa.tmX = a.tmB; wa.tmW = a.tmA; wa.tmW2 = a.tmA2; wa.sfw = a.sfa; wa.sfw2 = a.sfa2; wa.sfx = a.sfb; wa.ldsfx = ldsfb; wa.alpha = alpha; wa.alpha2 = alpha2;
+      wa.tiles = a.tiles; wa.n_tiles = n_tiles; wa.Y = Y; wa.R = a.R; wa.status = status; wa.q_out = a.q_out; wa.sf_out = a.sf_out; wa.inv_gs_out = inv_gs_out;
+      wa.ldsf_out = ldsf_out; wa.ldy = ldy; wa.rows_total = rows_total; wa.N = N; wa.K = K; wa.epi = epi; wa.act = act;
+      return ca_gemm_wide(kind, swiglu != 0, wa, items, stream);
     }
   }
   long long work = tiles ? (long long)max_tiles * n_nt : (long long)((rows_total + tn - 1) / tn) * n_nt * a.splits;

@@ -37,6 +37,7 @@ PREFILL_ATTN_MIN_Q = int(os.environ.get("CUTEAFD_PREFILL_ATTN_MIN_Q", "64"))
 # (265.3 vs 265.4 us per layer) and 0.6 % slower on the multi-GPU layouts (one block selects for every token instead of a block per token).
 FP8_FUSE_GATE_UP = os.environ.get("CUTEAFD_FP8_FUSE_GATE_UP", "1") != "0"      # FP8 dense FFNs: gate and up projections as one GEMM
 CLUSTER_KINDS = (KIND_BF16,) + tuple(FP4_KINDS)       # operand kinds with a cluster split-K kernel besides FP8
+WIDE_KINDS = (KIND_BF16,) + tuple(FP4_KINDS)          # expert kinds of the wide GEMM (csrc/tc_gemm_wide.cu)
 ROUTER_FUSED = os.environ.get("CUTEAFD_ROUTER_FUSED", "0") == "1"
 
 
@@ -110,10 +111,10 @@ class Lane:
         if m.n_experts and eng.n_local_experts:
             rows = cap * m.top_k
             exp_rows = max(1, math.ceil(rows / max(1, m.n_experts)) * 2)
-            # token tiles of the grouped expert GEMMs stay <= 32 rows even in prefill: those tiles run two CTAs per SM with
-            # double-buffered accumulators, which measured 2x faster end to end than 128-row tiles (one CTA per SM, the
-            # SwiGLU epilogue not overlapped); CUTEAFD_TNG overrides for experiments
-            self.tn_g = pick_tn(min(exp_rows, int(os.environ.get("CUTEAFD_TNG", "32"))), swiglu=True)
+            # token tiles of the grouped expert GEMMs: prompt-sized lanes take the wide kernel's 128 rows, smaller ones at most 32 (two CTAs
+            # per SM stream the weights); CUTEAFD_TNG overrides for experiments
+            wide = cap >= 1024 and ek in WIDE_KINDS
+            self.tn_g = 128 if wide and "CUTEAFD_TNG" not in os.environ else pick_tn(min(exp_rows, int(os.environ.get("CUTEAFD_TNG", "32"))), swiglu=True)
             self.max_tiles = eng.n_local_experts + rows // self.tn_g + 1
             self.router_logits = torch.zeros(cap, m.n_experts, dtype=torch.float32, device=dev)
             self.idx, self.wts = i32(cap, m.top_k), torch.zeros(cap, m.top_k, dtype=torch.float32, device=dev)
