@@ -435,13 +435,13 @@ class Engine:
             raise NotImplementedError("linear-attention layers run with bf16 dense projections")
         self._dense(lw.lin_ba, L.xn_act, b["ba"], T)
         st, n_seq = ptr(self.status), sh.n_seq
-        native.call("cuteafd_short_conv4_peek" if sv else "cuteafd_short_conv4", ptr(qkvz), ptr(lw.lin_conv), ptr(self.lin_carry[j]), ptr(md["state_slot"]),
-                    ptr(md["q_start"]), ptr(md["q_len"]), ptr(b["conv"]), n_seq, C, Nq, self.max_seqs, st, native.stream())
+        native.call("cuteafd_short_conv4_run", ptr(qkvz), ptr(lw.lin_conv), ptr(self.lin_carry[j]), ptr(md["state_slot"]),
+                    ptr(md["q_start"]), ptr(md["q_len"]), ptr(b["conv"]), n_seq, C, Nq, self.max_seqs, sh.max_q_len, 0 if sv else 1, st, native.stream())
         native.call("cuteafd_linear_prepare", ptr(b["conv"]), ptr(b["ba"]), ptr(lw.lin_a_log), ptr(lw.lin_dt_bias), ptr(b["q"]), ptr(k_), ptr(v_),
                     ptr(g_), ptr(beta_), T, Hk, Hv, b["ba"].shape[1], pc, native.stream())
-        native.call("cuteafd_gated_delta_step", ptr(b["q"]), ptr(k_), ptr(v_), ptr(g_), ptr(beta_), ptr(self.lin_state[j]),
+        native.call("cuteafd_gated_delta_run", ptr(b["q"]), ptr(k_), ptr(v_), ptr(g_), ptr(beta_), ptr(self.lin_state[j]),
                     ptr(md["state_slot"]), ptr(md["q_start"]), ptr(md["q_len"]), ptr(b["o"]), None, n_seq, Hv, pc | (2 if sv else 0),
-                    self.max_seqs, st, native.stream())
+                    self.max_seqs, sh.max_q_len, st, native.stream())
         native.call("cuteafd_gated_rmsnorm", ptr(b["o"]), ptr(qkvz), ptr(lw.lin_norm), ptr(b["on"]), T, Hv, Nq, C, spec.rms_eps, native.stream())
         self._attn_out(li, lw, b["on_act"], L, T)
         self.launches_per_step += 7
@@ -467,10 +467,10 @@ class Engine:
         b, save, st = L.lin_buf(self), L.lin_save(self), ptr(self.status)
         for j, li in enumerate(self.lin_layers):
             lw, sv = self.weights.layer(li), save[j]
-            native.call("cuteafd_short_conv4", ptr(sv["qkvz"]), ptr(lw.lin_conv), ptr(self.lin_carry[j]), ptr(md["state_slot"]), ptr(md["q_start"]),
-                        ptr(self._acc_dev), ptr(b["conv"]), sh.n_seq, C, Nq, self.max_seqs, st, native.stream())
-            native.call("cuteafd_gated_delta_step", ptr(sv["k"]), ptr(sv["k"]), ptr(sv["v"]), ptr(sv["g"]), ptr(sv["beta"]), ptr(self.lin_state[j]),
-                        ptr(md["state_slot"]), ptr(md["q_start"]), ptr(self._acc_dev), ptr(b["o"]), None, sh.n_seq, Hv, pc, self.max_seqs, st,
+            native.call("cuteafd_short_conv4_run", ptr(sv["qkvz"]), ptr(lw.lin_conv), ptr(self.lin_carry[j]), ptr(md["state_slot"]), ptr(md["q_start"]),
+                        ptr(self._acc_dev), ptr(b["conv"]), sh.n_seq, C, Nq, self.max_seqs, sh.max_q_len, 1, st, native.stream())
+            native.call("cuteafd_gated_delta_run", ptr(sv["k"]), ptr(sv["k"]), ptr(sv["v"]), ptr(sv["g"]), ptr(sv["beta"]), ptr(self.lin_state[j]),
+                        ptr(md["state_slot"]), ptr(md["q_start"]), ptr(self._acc_dev), ptr(b["o"]), None, sh.n_seq, Hv, pc, self.max_seqs, sh.max_q_len, st,
                         native.stream())
 
     def _attention_layer(self, li: int, lw: LayerWeights, L: Lane, sh: StepShape):

@@ -55,10 +55,12 @@ _PROTOS = {
     "cuteafd_tmap_encode_kv": [P, P, I, U64],
     "cuteafd_mla_attention": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, F, P, P],
     "cuteafd_tmap_encode_latent": [P, P, U64],
+    "cuteafd_gated_delta_run": [P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P, P],
     "cuteafd_gated_delta_step": [P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, P, P],
     "cuteafd_linear_prepare": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, P],
     "cuteafd_gated_rmsnorm": [P, P, P, P, I, I, I, I, F, P],
     "cuteafd_short_conv4": [P, P, P, P, P, P, P, I, I, I, I, P, P],
+    "cuteafd_short_conv4_run": [P, P, P, P, P, P, P, I, I, I, I, I, I, P, P],
     "cuteafd_short_conv4_peek": [P, P, P, P, P, P, P, I, I, I, I, P, P],
     "cuteafd_mhc_boundary": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, F, P],
     "cuteafd_vision_rgb_patches": [P, P, P, I, I, I, I, I, P],

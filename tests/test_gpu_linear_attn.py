@@ -71,3 +71,80 @@ def test_short_conv4_carries_its_history():
         assert status.tolist() == [0, 0, 0, 0]
         assert float((y.float().cpu() - want).abs().max()) < 2e-2
     assert bool((carry[0] == 0).all()) and bool((carry[2] == 0).all())
+
+
+@pytest.mark.parametrize("per_channel", [False, True])
+@pytest.mark.parametrize("lens", [(8, 7, 17), (64, 1, 200)])
+def test_long_runs_of_the_delta_rule_match_reference(per_channel, lens):
+    """Runs around the eight tokens that are staged at a time, with and without the state written back: the fp32 recurrence in the reference's order of
+    tokens; sums over 128 rows in another order."""
+    g = torch.Generator().manual_seed(sum(lens))
+    H, n_slots, T = 4, 3, sum(lens)
+    b16 = lambda t: t.to(torch.bfloat16)
+    q = b16(torch.nn.functional.normalize(torch.randn(T, H, 128, generator=g), dim=-1) * 128 ** -0.5)
+    k = b16(torch.nn.functional.normalize(torch.randn(T, H, 128, generator=g), dim=-1))
+    v = b16(torch.randn(T, H, 128, generator=g))
+    gate = torch.rand(T, H, 128, generator=g) * 0.2 + 0.8 if per_channel else torch.rand(T, H, generator=g) * 0.2 + 0.8
+    beta, state0 = torch.rand(T, H, generator=g), torch.randn(n_slots, H, 128, 128, generator=g) * 0.1
+    d = lambda t: t.to(DEV).contiguous()
+    i32 = lambda v_: torch.tensor(v_, dtype=torch.int32, device=DEV)
+    starts, slots = [0, lens[0], lens[0] + lens[1]], [1, 2, 0]
+    args = [d(t) for t in (q, k, v, gate, beta)]
+    meta, status = [i32(x) for x in (slots, starts, lens)], torch.zeros(4, dtype=torch.int32, device=DEV)
+    for keep, max_len in ((2, max(lens)), (0, max(lens)), (0, 0)):       # outputs only, with the state, length not known
+        state, out = d(state0.clone()), torch.zeros(T, H, 128, dtype=torch.bfloat16, device=DEV)
+        call("cuteafd_gated_delta_run", *map(ptr, args), ptr(state), *map(ptr, meta), ptr(out), None, 3, H, int(per_channel) | keep, n_slots, max_len, ptr(status), stream())
+        torch.cuda.synchronize()
+        assert status.tolist() == [0, 0, 0, 0]
+        for t0, n, slot in zip(starts, lens, slots):
+            rows = slice(t0, t0 + n)
+            want, final, _ = rops.gated_delta_rule(q[rows].float(), k[rows].float(), v[rows].float(), gate[rows], beta[rows], state0[slot])
+            # bf16 outputs: half a last place of the largest, 2^-9
+            assert float((out[rows].float().cpu() - want).abs().max()) < 2 ** -8 * float(want.abs().max())
+            assert torch.equal(state[slot].cpu(), state0[slot]) if keep else torch.allclose(state[slot].cpu(), final, atol=1e-5, rtol=1e-5)
+
+
+@pytest.mark.parametrize("per_channel", [False, True])
+def test_short_runs_of_many_sequences_equal_the_long_form(per_channel):
+    """Decode-sized steps of more sequences than one wave of the four-block form: the one-block form, against the other one."""
+    g = torch.Generator(device=DEV).manual_seed(5)
+    H, n, rows = 8, 20, 3
+    T = n * rows
+    b16 = lambda t: t.to(torch.bfloat16).contiguous()
+    unit = lambda: b16(torch.nn.functional.normalize(torch.randn(T, H, 128, generator=g, device=DEV), dim=-1))
+    args = [unit(), unit(), b16(torch.randn(T, H, 128, generator=g, device=DEV)),
+            torch.rand(*((T, H, 128) if per_channel else (T, H)), generator=g, device=DEV) * 0.3 + 0.7, torch.rand(T, H, generator=g, device=DEV)]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    meta = [i32(list(range(n))), i32([rows * s for s in range(n)]), i32([rows - s % 2 for s in range(n)])]
+    state0, status, got = torch.randn(n, H, 128, 128, generator=g, device=DEV) * 0.1, torch.zeros(4, dtype=torch.int32, device=DEV), []
+    for max_len in (rows, 0):
+        state, out = state0.clone(), torch.zeros(T, H, 128, dtype=torch.bfloat16, device=DEV)
+        call("cuteafd_gated_delta_run", *map(ptr, args), ptr(state), *map(ptr, meta), ptr(out), None, n, H, int(per_channel), n, max_len, ptr(status), stream())
+        got.append((state, out.float()))
+    torch.cuda.synchronize()
+    assert status.tolist() == [0, 0, 0, 0]
+    assert torch.allclose(got[0][0], got[1][0], atol=1e-5, rtol=1e-5)
+    assert float((got[0][1] - got[1][1]).abs().max()) <= 2 ** -8 * float(got[1][1].abs().max())      # a last place of bf16
+
+
+@pytest.mark.parametrize("C,ldx", [(384, 512), (130, 131)])          # 8-byte words, and odd rows
+@pytest.mark.parametrize("lens", [(1, 2, 3), (16, 17, 50), (4, 200, 33)])
+def test_short_conv4_in_token_blocks_matches_reference(C, ldx, lens):
+    """Sequences cut into blocks of 16 tokens, fewer blocks than the longest needs, the carry read and replaced by the same launch."""
+    g = torch.Generator().manual_seed(C + sum(lens))
+    T, n_slots = sum(lens), 4
+    b16 = lambda t: t.to(torch.bfloat16)
+    x, w, carry0 = b16(torch.randn(T, ldx, generator=g)), torch.randn(C, 4, generator=g) * 0.5, b16(torch.randn(n_slots, 3, C, generator=g))
+    i32 = lambda v_: torch.tensor(v_, dtype=torch.int32, device=DEV)
+    starts, slots = [0, lens[0], lens[0] + lens[1]], [3, 0, 2]
+    xd, wd, meta, status = x.to(DEV), w.to(DEV), [i32(t) for t in (slots, starts, lens)], torch.zeros(4, dtype=torch.int32, device=DEV)
+    for update, max_len in ((1, max(lens)), (1, 40), (0, max(lens)), (1, 0)):
+        carry, y = carry0.to(DEV), torch.zeros(T, C, dtype=torch.bfloat16, device=DEV)
+        call("cuteafd_short_conv4_run", ptr(xd), ptr(wd), ptr(carry), *map(ptr, meta), ptr(y), 3, C, ldx, n_slots, max_len, update, ptr(status), stream())
+        torch.cuda.synchronize()
+        assert status.tolist() == [0, 0, 0, 0]
+        for t0, n, slot in zip(starts, lens, slots):
+            want, after = rops.short_conv4(x[t0:t0 + n, :C].float(), w, carry0[slot].float())
+            assert float((y[t0:t0 + n].float().cpu() - want).abs().max()) < 2 ** -7 * float(want.abs().max())
+            assert torch.equal(carry[slot].cpu(), b16(after) if update else carry0[slot])
+        assert torch.equal(carry[1].cpu(), carry0[1])
