@@ -140,6 +140,19 @@ __device__ __forceinline__ uint8_t ue8m0_ceil(float s) {
   return (uint8_t)min(e, 254u);
 }
 
+// Eight E2M1 codes of values already divided by their block's scale, lowest nibble first: the conversion instruction rounds as float_to_e2m1
+// does; a value that rounds to zero loses its sign, as there.
+__device__ __forceinline__ uint32_t pack_e2m1x8(const float* v) {
+  uint32_t w;
+  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\tcvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n\tcvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\t"
+      "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
+      : "=r"(w) : "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]));
+  const uint32_t nonzero = (w | (w >> 1) | (w >> 2)) & 0x11111111u;
+  return w & (0x77777777u | (nonzero << 3));
+}
+
 // FP4 block quantisation of 8 consecutive values held by this thread.  The block (16 values NVFP4, 32 values MXFP4)
 // spans 2 or 4 adjacent lanes, which must call this together (full warp converged).  Returns the 8 packed E2M1
 // codes; `sb` is the block's scale byte (E4M3 with the static global scale 1/inv_gs, or UE8M0).  Same arithmetic as
@@ -162,10 +175,10 @@ __device__ __forceinline__ uint32_t quant8_fp4(const float* v, float inv_gs, uin
     eff = e4m3_to_float(sb) / inv_gs;
   }
   const float inv = eff > 0.f ? 1.f / eff : 0.f;
-  uint32_t w = 0;
+  float t[8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) w |= float_to_e2m1(v[j] * inv) << (4 * j);
-  return w;
+  for (int j = 0; j < 8; ++j) t[j] = v[j] * inv;
+  return pack_e2m1x8(t);
 }
 // Writes one thread's share of a quantised row: codes of elements [i, i+8) and, from the first lane of the block,
 // the scale byte.  qkind 1 = NVFP4, 2 = MXFP4.

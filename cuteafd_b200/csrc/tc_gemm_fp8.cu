@@ -420,11 +420,49 @@ __global__ void act_quant_fp8_block128_kernel(const bf16* __restrict__ x, uint8_
   if (lane == 0) sa[(size_t)r * nkb + g] = scale;
 }
 
+// The same for rows of whole 16-byte words: half a warp per group, eight channels per lane, four groups of every half in flight (a group per warp
+// and block churn bounded the form above: 50 us for 2048 rows of 16384, 33 us here).
+__global__ void __launch_bounds__(256) act_quant_fp8_block128x8_kernel(const bf16* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ sa, uint32_t groups, int K, int ldx,
+                                                                      uint32_t nkb) {
+  pdl_launch(); pdl_wait();
+  const uint32_t half = (blockIdx.x * blockDim.x + threadIdx.x) >> 4, lane = threadIdx.x & 15;
+  uint4 raw[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const uint32_t w = half * 4 + u, r = w / nkb, k0 = (w - r * nkb) * 128 + lane * 8;
+    raw[u] = w < groups && k0 < (uint32_t)K ? *(const uint4*)(x + (size_t)r * ldx + k0) : make_uint4(0u, 0u, 0u, 0u);
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const uint32_t w = half * 4 + u, r = w / nkb, g = w - r * nkb, k0 = g * 128 + lane * 8;
+    const bf16* e = (const bf16*)&raw[u];
+    float v[8], amax = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { v[j] = __bfloat162float(e[j]); amax = fmaxf(amax, fabsf(v[j])); }
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    const float scale = fmaxf(amax, 1e-4f) / 448.f;
+    if (w < groups) {
+      if (k0 < (uint32_t)K) {
+        uint32_t p[2] = {0u, 0u};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) p[j >> 2] |= (uint32_t)float_to_e4m3(v[j] / scale) << (8 * (j & 3));
+        *(uint2*)(q + (size_t)r * K + k0) = make_uint2(p[0], p[1]);
+      }
+      if (lane == 0) sa[(size_t)r * nkb + g] = scale;
+    }
+  }
+}
+
 extern "C" int cuteafd_act_quant_fp8_block128(const void* x, void* q, float* sa, int rows, int K, int ldx, cudaStream_t s) {
   CA_REQUIRE(K % 4 == 0 && ldx % 4 == 0, "act_quant_fp8_block128: K must be a multiple of 4");
   if (rows <= 0) return CA_OK;
   const int nkb = (K + 127) / 128;
   const long long warps = (long long)rows * nkb;
+  if (K % 8 == 0 && ldx % 8 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)q & 7) == 0 && warps > 4096 && warps < (1ll << 27)) {
+    CA_LAUNCH_PDL(act_quant_fp8_block128x8_kernel, (int)((warps + 63) / 64), 256, 0, s, (const bf16*)x, (uint8_t*)q, sa, (uint32_t)warps, K, ldx, (uint32_t)nkb);
+    return CA_OK;
+  }
   CA_LAUNCH_PDL(act_quant_fp8_block128_kernel, (int)((warps * 32 + 255) / 256), 256, 0, s, (const bf16*)x, (uint8_t*)q, sa, rows, K, ldx, nkb);
   return CA_OK;
 }

@@ -52,19 +52,6 @@ __device__ __forceinline__ void ld_32b(const void* p, uint32_t* w) {
 }
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) { const bf162 h = __floats2bfloat162_rn(a, b); return *(const uint32_t*)&h; }
 
-// Eight E2M1 codes of values already divided by their block's scale, lowest first; a value that rounds to zero loses its sign, as in
-// float_to_e2m1.
-__device__ __forceinline__ uint32_t pack_e2m1x8(const float* v) {
-  uint32_t w;
-  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\tcvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n\tcvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\t"
-      "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
-      : "=r"(w) : "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]));
-  const uint32_t nonzero = (w | (w >> 1) | (w >> 2)) & 0x11111111u;
-  return w & (0x77777777u | (nonzero << 3));
-}
-
 template <int KIND>
 __device__ __forceinline__ uint32_t wide_idesc(uint32_t sf_id) {
   uint32_t d = ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);

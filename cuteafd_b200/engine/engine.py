@@ -122,6 +122,8 @@ class Lane:
             self.counts, self.offsets = i32(eng.n_local_experts), i32(eng.n_local_experts)
             self.tiles, self.n_tiles, self.n_rows = i32(self.max_tiles, 4), i32(1), i32(1)
             self.xs = ActBuffer.alloc(ek, rows, H, self.tn_g, dev)
+            # prompt-sized lanes quantise every token once and gather bytes; small ones quantise while they gather (one launch less)
+            self.xt = ActBuffer.alloc(ek, cap, H, self.tn_g, dev) if wide and ek in FP4_KINDS and H % 32 == 0 else None
             self.h1 = bf(rows, m.intermediate)
             self.h1_q = (ActBuffer.alloc(ek, rows, m.intermediate, self.tn_g, dev) if ek != KIND_BF16
                          else ActBuffer.wrap_bf16(self.h1, self.tn_g))
@@ -505,16 +507,19 @@ class Engine:
         self.launches_per_step += 2 + (1 if sh.attn_splits > 1 else 0)
 
     _ffn_in_quantised = False
+    _tokens_quantised = False          # the FFN norm left the experts' operand of every token in the lane's `xt`
 
     def _ffn_norm(self, lw: LayerWeights, L: Lane, T: int):
         """RMSNorm in front of the FFN block -> L.xn (router, dispatch and gather read bf16 rows); when a dense or shared expert
         with FP8 operands follows, its quantised input is written by the same launch."""
         if self.spec.hyper_streams:
             self._hc_boundary(L, T, lw.hc_ffn, lw.ffn_norm)
-            self._ffn_in_quantised = False
+            self._ffn_in_quantised = self._tokens_quantised = False
             return
         fuse = L.xq.kind == KIND_FP8B and self.spec.hidden % 256 == 0 and lw.ws_gate is not None and lw.ws_gate.kind == KIND_FP8B
-        ops.add_rmsnorm(L.x, None, lw.ffn_norm, L.xn, self.spec.rms_eps, rows=T, quant=L.xq if fuse else None)
+        xt = getattr(L, "xt", None) if lw.w_gate is not None and not fuse and self.spec.hidden % 256 == 0 else None
+        self._tokens_quantised = xt is not None
+        ops.add_rmsnorm(L.x, None, lw.ffn_norm, L.xn, self.spec.rms_eps, rows=T, quant=L.xq if fuse else xt, inv_gs=lw.w_gate.inv_act_gs if xt is not None else None)
         self._ffn_in_quantised = fuse
         self.launches_per_step += 1
 
@@ -617,6 +622,11 @@ class Engine:
         rows = T * m.top_k
         if L.xs.kind == KIND_BF16:
             ops.gather_rows(L.xn, L.src_token, L.n_rows, L.xs.data, rows)
+        elif L.xt is not None:
+            if not self._tokens_quantised:
+                ops.quant_fp4_rows(L.xn, L.xt, rows=T, inv_gs=lw.w_gate.inv_act_gs)
+                self.launches_per_step += 1
+            ops.route_gather(L.xt.data, L.xt.sf, L.src_token, L.n_rows, L.xs, rows, status=self.status)
         else:
             ops.quant_fp4_rows(L.xn, L.xs, src_rows=L.src_token, n_rows_dev=L.n_rows, rows=rows, inv_gs=lw.w_gate.inv_act_gs)
         if L.h1_q.kind != KIND_BF16 and m.intermediate % 32 == 0:

@@ -399,7 +399,7 @@ class MlaEngine(Engine):
             self._pf_lat = torch.zeros(cap, DQK, dtype=torch.bfloat16, device=dev)
             self._pf_kvb = torch.zeros(cap, Hl * 256, dtype=torch.bfloat16, device=dev)
             view = self._pf_lat[:, :DV]
-            self._pf_act = ActBuffer(KIND_BF16, cap, DV, 256, view, ops.encode_tmap(view, 256))
+            self._pf_act = ActBuffer(KIND_BF16, cap, DV, 128, view, ops.encode_tmap(view, 128))        # the wide GEMM's token tiles
             self._pf_cap = cap
         st = ptr(self.status)
         call("cuteafd_mla_gather_ctx", ptr(self.kv[li]), ptr(md["page_table"]), ptr(self._pf_starts), ptr(md["kv_len"]), ptr(self._pf_lat), n_seq,
