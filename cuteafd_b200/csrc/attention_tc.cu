@@ -15,6 +15,10 @@
 // overlaps the other's MMAs and loads.  With several splits the unnormalised (O, m, l) partials go to scratch
 // and `attn_merge_kernel` (attention.cu) combines them.
 //
+// Steps of so many sequences that none is split, without a window, cut every sequence by ITS length (`plan_slot`): the launch has a fixed number of
+// slots, each block works out from the lengths which sequence and which part of it its slot is.  48 sequences of 100 to 9,900 tokens (64 query heads over 4):
+// one block each per head, 306 us, as long as the longest; now 150 us.
+//
 // Replaces the reference's sparse/GQA attention programs (AOT-exported, sources absent) and its wmma/mma.sync
 // kernels (native/shared/cuda/draft_attention.cu:41-340, families/glm5/cuda/glm_mla_prefill.cu:123-960).
 #include <string.h>
@@ -42,6 +46,8 @@ struct AttnTcArgs {
   float* part_ml;
   int* status;
   int q_stride, Hq, Hkv, max_pages, n_splits, window, max_q_tiles, T;
+  int slots, n_seq, wave, max_q; // slots > 0: parts by length; blocks per head and query tile that run at once; longest query run
+  int4* slot_of_row;            // ... and what the merge needs: {first slot, number of slots, row within its sequence} of every query row
   int v_head0, dv, ldo;         // value width of the output (at most VC * 64) and its row pitch: head h at column h * dv
   float scale;
 };
@@ -66,6 +72,41 @@ __device__ __forceinline__ void tmem_st_x16(uint32_t addr, const uint32_t* r) {
                  "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// What slot `slot` of a step holds.  Sequences of uneven length are cut into pieces of about L pages, so many that all pieces fit the slots
+// (sum ceil(p / L) <= n_seq + sum p / L); even ones are left whole (a wave of pieces plus a piece's start-up must be shorter than the longest
+// sequence).  All pieces of a sequence share the reference maximum of its first page (each looks at that page once more), so probabilities are
+// rounded alike however a sequence is cut and only the order of fp32 sums depends on it.  Every lane of the warp must call it.
+struct SlotPlan { int seq, piece, cuts; };               // sequence (-1: the slot is not used), piece of it, its number of pieces
+__device__ __forceinline__ SlotPlan plan_slot(const AttnTcArgs& a, int slot) {
+  const int lane = threadIdx.x & 31;
+  auto pages_of = [&](int s) { return s < a.n_seq ? (a.kv_len[s] + APAGE - 1) / APAGE : 0; };
+  int total = 0, longest = 0;
+  for (int s0 = 0; s0 < a.n_seq; s0 += 32) {
+    const int p = pages_of(s0 + lane);
+    total += p; longest = max(longest, p);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) { total += __shfl_xor_sync(0xffffffffu, total, o); longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o)); }
+  const int room = a.slots - a.n_seq, L = max(4, (total + room - 1) / room);
+  const bool uneven = (total / a.wave + L + 4) * 10 < longest * 9;
+  SlotPlan r = {-1, 0, 1};
+  int base = 0;
+  for (int s0 = 0; s0 < a.n_seq && r.seq < 0; s0 += 32) {
+    const int cuts = s0 + lane < a.n_seq ? (uneven ? max(1, (pages_of(s0 + lane) + L - 1) / L) : 1) : 0;
+    int end = cuts;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, end, o); if (lane >= o) end += v; }
+    end += base;
+    const uint32_t hit = __ballot_sync(0xffffffffu, slot < end && slot >= end - cuts);
+    if (hit) {
+      const int w = __ffs(hit) - 1;
+      r.seq = s0 + w; r.cuts = __shfl_sync(0xffffffffu, cuts, w); r.piece = slot - __shfl_sync(0xffffffffu, end - cuts, w);
+    }
+    base = __shfl_sync(0xffffffffu, end, 31);
+  }
+  return r;
+}
 
 template <int KC, int VC>
 struct AttnTcCfg {
@@ -99,8 +140,14 @@ __global__ void __launch_bounds__(192, AttnTcCfg<KC, VC>::OCC) paged_attn_tc_ker
 
   const int G = a.Hq / a.Hkv;
   const int tok_per_tile = 128 / G;
-  const int split = blockIdx.x, kvh = blockIdx.y;
-  const int seq = blockIdx.z / a.max_q_tiles, qt = blockIdx.z % a.max_q_tiles;
+  const int kvh = blockIdx.y;
+  int split = blockIdx.x, n_splits = a.n_splits, seq = blockIdx.z / a.max_q_tiles, qt = blockIdx.z % a.max_q_tiles;
+  if (a.slots) {
+    const SlotPlan p = plan_slot(a, blockIdx.x);
+    if (p.seq < 0) return;
+    seq = p.seq; split = p.piece; n_splits = p.cuts; qt = blockIdx.z;
+  }
+  const bool direct = !a.slots && n_splits == 1;        // else partials for the merge
   const int qlen = a.q_len[seq], kvlen = a.kv_len[seq];
   const int tok0 = qt * tok_per_tile;
   if (tok0 >= qlen) return;
@@ -113,14 +160,17 @@ __global__ void __launch_bounds__(192, AttnTcCfg<KC, VC>::OCC) paged_attn_tc_ker
   const int first_page = lo / APAGE, last_page = (hi + APAGE - 1) / APAGE;
   // the pages that count: those of kept first keys (or tiles of pooled blocks) in front of the window, then the window's; a split takes a run of them
   const int kept = a.x.lead_tiles(first_page, APAGE, hi - 1, a.window), n_pages = kept + last_page - first_page;
-  const int per = (n_pages + a.n_splits - 1) / a.n_splits;
+  const int per = (n_pages + n_splits - 1) / n_splits;
   const int p0 = split * per, p1 = min(n_pages, p0 + per);
-  const int n_tiles = max(0, p1 - p0);
-  auto page_at = [&](int i) { const int j = p0 + i; return j < kept ? j : j - kept + first_page; };
-  auto pooled_at = [&](int i) { return a.x.pool > 0 && p0 + i < kept; };
+  // a piece behind the first one starts with the sequence's first page, which only sets the reference maximum
+  const bool lead = a.slots && p0 > 0 && p1 > p0;
+  const int n_tiles = max(0, p1 - p0) + (lead ? 1 : 0), tile0 = lead ? p0 - 1 : p0;
+  auto page_at = [&](int i) { const int j = lead && i == 0 ? 0 : tile0 + i; return j < kept ? j : j - kept + first_page; };
+  auto pooled_at = [&](int i) { return a.x.pool > 0 && tile0 + i < kept; };
 
   // Decode-shaped tiles (<= 32 real rows) replicate the rows into every 32-lane quarter of the MMA tile so that
   // the four softmax warps each take 16 of the 64 score columns of the SAME rows (4x shorter per-tile chain).
+  if (a.slots && split == 0 && kvh == 0 && tid < ntok) a.slot_of_row[row_base + tid] = make_int4((int)blockIdx.x, n_splits, tok0 + tid, 0);
   const bool rep4 = R <= 32;
   const int n_live_warps = rep4 ? 4 : (R + 31) / 32;    // softmax warps with work
   if (tid == 0) {
@@ -291,12 +341,13 @@ __global__ void __launch_bounds__(192, AttnTcCfg<KC, VC>::OCC) paged_attn_tc_ker
           }
           tc_wait_st();
         }
+        const bool none = m_ref == -INFINITY || (lead && i == 0);      // no probabilities: nothing seen yet, or the page that only sets the reference
         uint32_t pk[8];
         float psum = 0.f;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const float a0 = __uint_as_float(sr[2 * j]), a1 = __uint_as_float(sr[2 * j + 1]);
-          const float e0 = (m_ref == -INFINITY) ? 0.f : exp2f(a0 - m_ref), e1 = (m_ref == -INFINITY) ? 0.f : exp2f(a1 - m_ref);
+          const float e0 = none ? 0.f : exp2f(a0 - m_ref), e1 = none ? 0.f : exp2f(a1 - m_ref);
           psum += e0 + e1;
           bf162 h = __floats2bfloat162_rn(e0, e1);
           pk[j] = *(uint32_t*)&h;
@@ -355,12 +406,13 @@ __global__ void __launch_bounds__(192, AttnTcCfg<KC, VC>::OCC) paged_attn_tc_ker
         }
         tc_wait_st();
       }
+      const bool none = m_ref == -INFINITY || (lead && i == 0);
       float psum = 0.f;
       uint32_t pk[32];
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
         const float a0 = __uint_as_float(sr[2 * j]), a1 = __uint_as_float(sr[2 * j + 1]);
-        const float e0 = (m_ref == -INFINITY) ? 0.f : exp2f(a0 - m_ref), e1 = (m_ref == -INFINITY) ? 0.f : exp2f(a1 - m_ref);
+        const float e0 = none ? 0.f : exp2f(a0 - m_ref), e1 = none ? 0.f : exp2f(a1 - m_ref);
         psum += e0 + e1;
         bf162 h = __floats2bfloat162_rn(e0, e1);
         pk[j] = *(uint32_t*)&h;
@@ -382,16 +434,17 @@ __global__ void __launch_bounds__(192, AttnTcCfg<KC, VC>::OCC) paged_attn_tc_ker
       const int t = row_base + rr / G, h = kvh * G + rr % G;
       const float m_nat = (m_ref == -INFINITY) ? -INFINITY : m_ref * 0.6931471805599453f;
       float scale_o = 1.f, lt = l;
-      if (a.n_splits == 1 && a.x.sink) {
+      if (direct && a.x.sink) {
         const float sk = a.x.sink[h], m2 = fmaxf(m_nat, sk);
         const float e1 = (m_nat == -INFINITY) ? 0.f : __expf(m_nat - m2);
         lt = l * e1 + __expf(sk - m2); scale_o = e1;
       }
-      const float inv = (lt > 0.f ? scale_o / lt : 0.f) * (a.n_splits == 1 ? a.x.head_factor(t, h) : 1.f);      // splits: the merge applies it
+      const float inv = (lt > 0.f ? scale_o / lt : 0.f) * (direct ? a.x.head_factor(t, h) : 1.f);      // splits: the merge applies it
       const bool gated = a.x.gate && a.x.gate_values;
       bf16* dst = a.out + (size_t)t * a.ldo + (size_t)h * a.dv;
       const bool vec = ((a.dv | a.ldo) & 7) == 0;      // otherwise heads do not start on 16 bytes
-      float* po = a.n_splits > 1 ? a.part_o + (((size_t)split * a.T + t) * a.Hq + h) * (VC * 64) : nullptr;
+      const size_t prow = (a.slots ? (size_t)blockIdx.x * a.max_q + (tok0 + rr / G) : (size_t)split * a.T + t) * a.Hq + h;
+      float* po = direct ? nullptr : a.part_o + prow * (VC * 64);
 #pragma unroll 1
       for (int c = 0; c < VC * 4; ++c) {
         uint32_t o[16];
@@ -401,7 +454,7 @@ __global__ void __launch_bounds__(192, AttnTcCfg<KC, VC>::OCC) paged_attn_tc_ker
           for (int j = 0; j < 16; ++j) o[j] = 0;
         }
         if (!live) continue;
-        if (a.n_splits == 1) {
+        if (direct) {
           if (gated) {
 #pragma unroll
             for (int j = 0; j < 16; ++j)
@@ -423,8 +476,8 @@ __global__ void __launch_bounds__(192, AttnTcCfg<KC, VC>::OCC) paged_attn_tc_ker
           for (int j = 0; j < 4; ++j) *(uint4*)(po + c * 16 + j * 4) = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
         }
       }
-      if (live && a.n_splits > 1) {
-        float* ml = a.part_ml + (((size_t)split * a.T + t) * a.Hq + h) * 2;
+      if (live && !direct) {
+        float* ml = a.part_ml + prow * 2;
         ml[0] = m_nat; ml[1] = l;
       }
     }
@@ -453,7 +506,7 @@ static int launch_attn_tc(const AttnTcArgs& a, int n_seq, cudaStream_t s) {
   }
   // No pre-fill of the (m, l) partials: every CTA writes them for all of its live rows, also when its split
   // holds no key (m = -inf, l = 0), and a CTA that gives up reports through the status word.
-  CA_LAUNCH_PDL((paged_attn_tc_kernel<KC, VC>), dim3(a.n_splits, a.Hkv, n_seq * a.max_q_tiles), 192, smem, s, a);
+  CA_LAUNCH_PDL((paged_attn_tc_kernel<KC, VC>), a.slots ? dim3(a.slots, a.Hkv, a.max_q_tiles) : dim3(a.n_splits, a.Hkv, n_seq * a.max_q_tiles), 192, smem, s, a);
   CA_CHECK_LAUNCH("paged_attention_tc");
   return CA_OK;
 }
@@ -473,7 +526,7 @@ extern "C" int cuteafd_attn_merge(const float* part_o, const float* part_ml, con
   CA_REQUIRE(part_o && part_ml && out && n_parts >= 1, "attn_merge: needs partials");
   if (T <= 0) return CA_OK;
   CA_LAUNCH_PDL(attn_merge8_kernel, dim3(T, (Hq * AD / 8 + 127) / 128), 128, 0, s, part_o, part_ml, sink_only(sink), (bf16*)out, T, Hq, (int)AD, (int)AD, Hq * AD, n_parts,
-                (uint8_t*)nullptr, (uint8_t*)nullptr, 0, (const float*)nullptr, 0);
+                (uint8_t*)nullptr, (uint8_t*)nullptr, 0, (const float*)nullptr, 0, (const int4*)nullptr, 0);
   CA_CHECK_LAUNCH("attn_merge");
   return CA_OK;
 }
@@ -493,7 +546,7 @@ extern "C" int cuteafd_paged_attention_tc(const void* q, const void* kv_map, con
   g_partials_only = false;
   CA_REQUIRE(!partials_only || n_splits >= 2, "paged_attention_tc: partials-only needs at least two splits");
   if (T <= 0 || n_seq <= 0) return CA_OK;
-  AttnTcArgs a;
+  AttnTcArgs a = {};
   a.q = (const bf16*)q; a.k_map = a.v_map = (const CUtensorMap*)kv_map; a.v_head0 = Hkv; a.dv = AD; a.ldo = Hq * AD; a.page_table = page_table; a.kv_len = kv_len; a.q_start = q_start;
   a.q_len = q_len; a.x = sink_only(sink); a.out = (bf16*)out; a.part_o = part_o; a.part_ml = part_ml; a.status = status;
   a.q_stride = q_stride; a.Hq = Hq; a.Hkv = Hkv; a.max_pages = max_pages; a.n_splits = n_splits; a.window = window; a.T = T; a.scale = scale;
@@ -503,9 +556,46 @@ extern "C" int cuteafd_paged_attention_tc(const void* q, const void* kv_map, con
   if (rc != CA_OK) return rc;
   if (n_splits > 1 && !partials_only) {
     CA_LAUNCH_PDL(attn_merge8_kernel, dim3(T, (Hq * AD / 8 + 127) / 128), 128, 0, s, part_o, part_ml, sink_only(sink), (bf16*)out, T, Hq, (int)AD, (int)AD, Hq * AD, n_splits,
-                  (uint8_t*)q_out, (uint8_t*)sf_out, ldsf, inv_gs, qkind);
+                  (uint8_t*)q_out, (uint8_t*)sf_out, ldsf, inv_gs, qkind, (const int4*)nullptr, 0);
     CA_CHECK_LAUNCH("attn_merge");
   }
+  return CA_OK;
+}
+
+// Slots of a step of `n_seq` sequences for the form below: one per sequence, and a wave and a half of blocks for further pieces.  Returns 0 where
+// it does not apply: a step that is split evenly fills a wave already (16 sequences of 4,096 in 4 parts: the plan and the unused slots cost 5 us of
+// 45), and one sequence is always even.
+extern "C" int cuteafd_attn_slots(int n_seq, int max_q_len, int Hq, int Hkv, int n_splits) {
+  if (n_seq < 2 || n_splits != 1 || max_q_len < 1 || max_q_len > 16 || Hkv < 1 || Hq % Hkv || 128 % (Hq / Hkv)) return 0;
+  const int tpt = 128 / (Hq / Hkv), tiles = (max_q_len + tpt - 1) / tpt;
+  const int wave = 2 * ca_sm_count() / (Hkv * tiles) > 1 ? 2 * ca_sm_count() / (Hkv * tiles) : 1;
+  return n_seq + wave + wave / 2 + 1;
+}
+
+// The same attention (no window) with every sequence split by its length.  part_o / part_ml hold `slots` (cuteafd_attn_slots) x max_q_len rows of Hq
+// partials, slot_of_row int4 [T].
+extern "C" int cuteafd_paged_attention_slots(const void* q, const void* kv_map, const int* page_table, const int* kv_len, const int* q_start, const int* q_len,
+                                             const float* sink, void* out, float* part_o, float* part_ml, void* slot_of_row, int T, int n_seq, int max_q_len, int q_stride,
+                                             int Hq, int Hkv, int max_pages, int slots, float scale, int* status, void* q_out, void* sf_out, int ldsf,
+                                             const float* inv_gs, int qkind, cudaStream_t s) {
+  CA_REQUIRE(qkind == 0 || (q_out && sf_out && (Hq * AD) % 256 == 0), "paged_attention_slots: FP4 output needs buffers and Hq*128 %% 256 == 0");
+  CA_REQUIRE(part_o && part_ml && slot_of_row && ((uintptr_t)slot_of_row & 15) == 0, "paged_attention_slots: needs scratch");
+  CA_REQUIRE(slots > 0 && slots == cuteafd_attn_slots(n_seq, max_q_len, Hq, Hkv, 1), "paged_attention_slots: %d slots", slots);
+  CA_REQUIRE(q_stride % 8 == 0, "paged_attention_slots: q rows must be 16-byte aligned");
+  if (T <= 0) return CA_OK;
+  AttnTcArgs a = {};
+  a.q = (const bf16*)q; a.k_map = a.v_map = (const CUtensorMap*)kv_map; a.v_head0 = Hkv; a.dv = AD; a.ldo = Hq * AD; a.page_table = page_table; a.kv_len = kv_len; a.q_start = q_start;
+  a.q_len = q_len; a.x = sink_only(sink); a.out = (bf16*)out; a.part_o = part_o; a.part_ml = part_ml; a.status = status;
+  a.q_stride = q_stride; a.Hq = Hq; a.Hkv = Hkv; a.max_pages = max_pages; a.n_splits = 1; a.T = T; a.scale = scale;
+  const int tpt = 128 / (Hq / Hkv);
+  a.max_q_tiles = (max_q_len + tpt - 1) / tpt;
+  a.slots = slots; a.n_seq = n_seq; a.max_q = max_q_len; a.slot_of_row = (int4*)slot_of_row;
+  a.wave = 2 * ca_sm_count() / (Hkv * a.max_q_tiles) > 1 ? 2 * ca_sm_count() / (Hkv * a.max_q_tiles) : 1;
+  const int rc = launch_attn_tc<2, 2>(a, n_seq, s);
+  if (rc != CA_OK) return rc;
+  CA_LAUNCH_PDL(attn_merge8_kernel, dim3(T, (Hq * AD / 8 + 127) / 128), 128, 0, s, part_o, part_ml, sink_only(sink), (bf16*)out, T, Hq, (int)AD, (int)AD, Hq * AD, 1,
+                (uint8_t*)q_out, (uint8_t*)sf_out, ldsf, inv_gs, qkind, (const int4*)slot_of_row, max_q_len);
+  CA_CHECK_LAUNCH("attn_merge");
   return CA_OK;
 }
 
@@ -548,7 +638,7 @@ extern "C" int cuteafd_window_attention(const void* q, const void* maps, const i
   if (rc != CA_OK) return rc;
   if (n_splits > 1) {
     CA_LAUNCH_PDL(attn_merge8_kernel, dim3(T, (Hq * dv_pad / 8 + 127) / 128), 128, 0, s, part_o, part_ml, a.x, (bf16*)out, T, Hq, dv_pad, dv, ldo, n_splits,
-                  (uint8_t*)nullptr, (uint8_t*)nullptr, 0, (const float*)nullptr, 0);
+                  (uint8_t*)nullptr, (uint8_t*)nullptr, 0, (const float*)nullptr, 0, (const int4*)nullptr, 0);
     CA_CHECK_LAUNCH("attn_merge");
   }
   return CA_OK;

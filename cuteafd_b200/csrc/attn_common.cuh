@@ -31,7 +31,9 @@ static __global__ void attn_merge_kernel(const float* __restrict__ part_o, const
 // output projection that follows (qkind 1 NVFP4 / 2 MXFP4; needs Hq * D % 256 == 0).  grid (T, ceil(Hq * D / 8 / 128)).
 static __global__ void attn_merge8_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, const AttnExtras<bf16> x,
                                           bf16* __restrict__ out, int T, int Hq, int D, int Dout, int ldo, int n_splits, uint8_t* __restrict__ q,
-                                          uint8_t* __restrict__ sf, int ldsf, const float* __restrict__ inv_gs_ptr, int qkind) {
+                                          uint8_t* __restrict__ sf, int ldsf, const float* __restrict__ inv_gs_ptr, int qkind, const int4* __restrict__ slots, int max_q) {
+  // `slots` (null: every row has n_splits partials): {first partial, number of partials, row within its sequence} of every query row, whose
+  // partials lie [partial][max_q][Hq].
   pdl_launch(); pdl_wait();
   const int t = blockIdx.x, vi = blockIdx.y * blockDim.x + threadIdx.x, vpr = D / 8;
   if (vi >= Hq * vpr) return;                     // whole warps leave together (Hq * D / 8 is a multiple of 32 with FP4 output)
@@ -39,6 +41,8 @@ static __global__ void attn_merge8_kernel(const float* __restrict__ part_o, cons
   // Up to eight splits at a time, every load issued before the first use: the (m, l) pairs and the partial rows of all splits are
   // in flight together (a loop that reads m, branches, then loads the row is one L2 round trip per split on a decode step's
   // critical path).  Partial rows of empty splits (m = -inf) are loaded but not used; the buffers always cover every split.
+  int first = 0, qrow = t, pitch = T;
+  if (slots) { const int4 m = slots[t]; first = m.x; n_splits = m.y; qrow = m.z; pitch = max_q; }
   const float sk = x.sink ? x.sink[h] : -INFINITY;
   float M = sk, L = 0.f;
   float o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -47,7 +51,7 @@ static __global__ void attn_merge8_kernel(const float* __restrict__ part_o, cons
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int s = min(s0 + j, n_splits - 1);
-      const size_t row = ((size_t)s * T + t) * Hq + h;
+      const size_t row = ((size_t)(first + s) * pitch + qrow) * Hq + h;
       ml[j] = *(const float2*)(part_ml + row * 2);
       const float4* po = (const float4*)(part_o + row * D + d0);
       pa[j] = po[0]; pb[j] = po[1];

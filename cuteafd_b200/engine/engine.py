@@ -485,13 +485,18 @@ class Engine:
         window = spec.layer_window(li)                # hybrid stacks: full and sliding-window layers differ in window, sink and theta
         ops.qk_norm_rope_kvwrite(L.qkv, md["positions"], md["slot_map"], lw.q_norm, lw.k_norm, self.kv[li], T,
                                  a.n_heads, a.n_kv_heads, a.head_dim, spec.layer_rope_theta(li), a.rope_interleaved, spec.rms_eps, self.status)
-        fused_q = False
+        fused_q, slots = False, 0 if window else self._attn_slots(sh)
         if self.kv_tmaps is not None and sh.attn_splits == 1 and sh.max_q_len >= PREFILL_ATTN_MIN_Q > 0:
             # prefill chunks: 128-key tiles with the query tile in tensor memory (8 + 8 tcgen05.mma per 128 keys instead of
             # 2 x (8 + 4) of the 64-key decode kernel)
             native.call("cuteafd_gqa_prefill_attention", ptr(L.qkv), ptr(self.kv_tmaps[li]), ptr(md["page_table"]), ptr(md["kv_len"]), ptr(md["q_start"]),
                         ptr(md["q_len"]), ptr(lw.sink), ptr(L.attn), T, sh.n_seq, sh.max_q_len, L.qkv.shape[1], a.n_heads, a.n_kv_heads,
                         md["page_table"].shape[1], window, a.head_dim ** -0.5, ptr(self.status), native.stream())
+        elif slots:
+            fused_q = ops.paged_attention_slots(L.qkv, self.kv_tmaps[li], md["page_table"], md["kv_len"], md["q_start"], md["q_len"], L.attn, T=T, n_seq=sh.n_seq,
+                                                max_q_len=sh.max_q_len, q_stride=L.qkv.shape[1], Hq=a.n_heads, Hkv=a.n_kv_heads,
+                                                slots=slots, part_o=self.part_o, part_ml=self.part_ml, slot_of_row=self.part_rows, sink=lw.sink,
+                                                status=self.status, quant=L.attn_q, inv_gs=lw.wo.inv_act_gs)
         elif self.kv_tmaps is not None:
             fused_q = ops.paged_attention_tc(L.qkv, self.kv_tmaps[li], md["page_table"], md["kv_len"], md["q_start"], md["q_len"], L.attn,
                                              T=T, n_seq=sh.n_seq, max_q_len=sh.max_q_len, q_stride=L.qkv.shape[1], Hq=a.n_heads,
@@ -504,7 +509,7 @@ class Engine:
                                 window=window, sink=lw.sink)
         oq = L.attn_q if fused_q else self._quant(L.attn, L.attn_q, T, lw.wo.inv_act_gs)
         self._attn_out(li, lw, oq, L, T)
-        self.launches_per_step += 2 + (1 if sh.attn_splits > 1 else 0)
+        self.launches_per_step += 2 + (1 if sh.attn_splits > 1 or slots else 0)
 
     _ffn_in_quantised = False
     _tokens_quantised = False          # the FFN norm left the experts' operand of every token in the lane's `xt`
@@ -706,13 +711,24 @@ class Engine:
             self.launches_per_step += 4
         return L
 
+    def _attn_slots(self, sh: StepShape) -> int:
+        """Blocks per head that cut the step's sequences by their lengths (0: every sequence into `attn_splits`)."""
+        a = self.spec.attn
+        return ops.attn_slots(sh.n_seq, sh.max_q_len, a.n_heads, a.n_kv_heads, sh.attn_splits) if a.kind == "gqa" and self.kv_tmaps is not None else 0
+
     def _ensure_attn_scratch(self, sh: StepShape):
         a, T = self.spec.attn, sh.T
-        if sh.attn_splits > 1:
-            need = sh.attn_splits * T * a.n_heads
+        slots = self._attn_slots(sh)
+        rows = max(sh.attn_splits * T if sh.attn_splits > 1 else 0, slots * sh.max_q_len)
+        if rows:
+            need = rows * a.n_heads
             if getattr(self, "part_o", None) is None or self.part_o.numel() < need * a.head_dim:
+                self._part_keep = getattr(self, "_part_keep", []) + [(getattr(self, "part_o", None), getattr(self, "part_ml", None))]     # captured steps hold them
                 self.part_o = torch.empty(need * a.head_dim, dtype=torch.float32, device=self.device)
                 self.part_ml = torch.empty(need * 2, dtype=torch.float32, device=self.device)
+            if slots and (getattr(self, "part_rows", None) is None or self.part_rows.shape[0] < T):
+                self._part_keep = getattr(self, "_part_keep", []) + [getattr(self, "part_rows", None)]
+                self.part_rows = torch.zeros(max(T, 256), 4, dtype=torch.int32, device=self.device)
         elif getattr(self, "part_o", None) is None:
             self.part_o = self.part_ml = None
 
