@@ -12,11 +12,13 @@
 // rows (columns 512..575); k_nope and V come from the expanded buffer [rows, Hl * 256] (per head: 128 key columns, then 128
 // value columns).  Both buffers are contiguous per sequence (`ctx_start[seq]` + key index), so tiles need no page table.
 //
-// Structure (one CTA per SM, 192 threads): warp 0 streams K tiles (48 KB, two stages) and V tiles (32 KB, two stages) by TMA;
+// Structure (one CTA per SM, 320 threads): warp 0 streams K tiles (48 KB, two stages) and V tiles (32 KB, two stages) by TMA;
 // the 128 x 192 query tile sits in tensor memory (96 columns) as the A operand of the score MMAs, which leaves the shared
-// memory to the K / V rings; warp 1 issues the MMAs (scores double-buffered in tensor memory), warps 2-5
-// run the softmax, one thread per row in two passes over the tile's 128 score columns (maximum, then exponentials, which
-// are computed BEFORE the wait for the PV product of tile i - 1, so that product runs under them).
+// memory to the K / V rings; warp 1 issues the MMAs (scores double-buffered in tensor memory), warps 2-9
+// run the softmax, two threads per row, each in two passes over half of the tile's 128 score columns (maximum, which the two exchange
+// through shared memory, then exponentials, which are computed BEFORE the wait for the PV product of tile i - 1, so that product runs
+// under them).  With one thread per row a tile's softmax was a single warp's chain per scheduler and bounded the loop:
+// 2048 rows over 8192 keys of 128 heads 1600 us, 1360 now; 4096 rows of 64 heads over 4 (the paged form below) 834 and 608.
 // Every wait is bounded and reports through the status word.
 //
 // Reference: the dedicated MLA prefill kernels of the GLM5 family (native/families/glm5/cuda/glm_mla_prefill.cu:123, 539),
@@ -31,6 +33,8 @@
 #define PF_NS 2                   // K stages
 #define PF_NSV 2                  // V stages
 #define PF_Q_BYTES 0              // the query tile lives in tensor memory (A operand of the score MMAs)
+#define PF_THREADS 320            // producer, MMA issuer, 2 x 4 softmax warps
+#define PF_TAIL 2304              // barriers (256 bytes), row maxima of the two halves of a tile (2 x 2 x 128 floats)
 #define PF_P_BYTES 32768          // 2 chunks (64 keys each) x [128 rows x 128 B]
 #define PF_V_STAGE 32768          // 2 chunks (64 dims each) x [128 keys x 128 B]
 
@@ -62,6 +66,8 @@ __device__ __forceinline__ uint64_t pf_desc_mn_sw128(uint32_t saddr, uint32_t lb
   d |= (uint64_t)2 << 61;
   return d;
 }
+// 2^x; results below 2^-126 are 0 (exp2f spends three more instructions on them)
+__device__ __forceinline__ float pf_exp2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 __device__ __forceinline__ uint32_t pf_idesc(int n, int b_mn_major) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)b_mn_major << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
@@ -74,7 +80,7 @@ __device__ __forceinline__ void pf_tmem_st_x16(uint32_t addr, const uint32_t* r)
 // KN 64-wide chunks of per-head key columns, KR rotated chunks shared by the heads (0 = attention without positions), NV chunks of value
 // columns; the expanded buffer holds (KN + NV) * 64 columns per head.  DeepSeek-V3: 2, 1, 2.
 template <int KN, int KR, int NV>
-__global__ void __launch_bounds__(192, 1) mla_prefill_kernel(const __grid_constant__ MlaPrefillArgs a) {
+__global__ void __launch_bounds__(PF_THREADS, 1) mla_prefill_kernel(const __grid_constant__ MlaPrefillArgs a) {
   pdl_launch(); pdl_wait();
   constexpr int NK = KN + KR, K_STAGE = NK * 16384, V_STAGE = NV * 16384, HEAD_W = (KN + NV) * 64;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -88,8 +94,11 @@ __global__ void __launch_bounds__(192, 1) mla_prefill_kernel(const __grid_consta
   uint64_t& p_full = bars[12]; uint64_t& o_done = bars[13];
   uint32_t& tmem_slot = *(uint32_t*)(bars + 14);
   int& abort_flag = *(int*)(bars + 15);
+  uint64_t* x_bar = bars + 16;          // [4]: the two softmax warps of a lane quarter
+  float* xchg = (float*)(bars + 32);    // [2][2][128]
   if (smem_u32(smem) & 1023) { if (threadIdx.x == 0) ca_dev_fail(a.status, CA_DEV_BAD_INDEX, 0xA13); return; }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+  const int hf = (warp - 2) >> 2;       // softmax warps: which half of a tile's score columns (and of the output columns)
 
   // the heaviest query tiles (most visible keys) are scheduled first
   const int head = blockIdx.x;
@@ -106,8 +115,9 @@ __global__ void __launch_bounds__(192, 1) mla_prefill_kernel(const __grid_consta
 
   if (tid == 0) {
     for (int s = 0; s < 2; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
-    for (int s = 0; s < 2; ++s) { mbar_init(&s_full[s], 1); mbar_init(&s_free[s], 128); }
-    mbar_init(&p_full, 128); mbar_init(&o_done, 1);
+    for (int s = 0; s < 2; ++s) { mbar_init(&s_full[s], 1); mbar_init(&s_free[s], 256); }
+    for (int s = 0; s < 4; ++s) mbar_init(&x_bar[s], 64);
+    mbar_init(&p_full, 256); mbar_init(&o_done, 1);
     abort_flag = 0;
     fence_barrier_init();
   }
@@ -126,7 +136,7 @@ __global__ void __launch_bounds__(192, 1) mla_prefill_kernel(const __grid_consta
     const bf16* src_nope = a.q_nope + ((size_t)head * a.ldt + t) * (KN * 64);
     const bf16* src_rope = a.q_rope + (size_t)t * a.qr_t + (size_t)head * a.qr_h;
 #pragma unroll 1
-    for (int g = 0; g < 2 * NK; ++g) {             // 16 columns = 32 elements per store
+    for (int g = hf * NK; g < (hf + 1) * NK; ++g) {             // 16 columns = 32 elements per store
       const bf16* src = (KR == 0 || g < 2 * KN) ? src_nope + g * 32 : src_rope + (g - 2 * KN) * 32;
       uint32_t w[16];
 #pragma unroll
@@ -213,29 +223,42 @@ __global__ void __launch_bounds__(192, 1) mla_prefill_kernel(const __grid_consta
       if (i + 2 < n_tiles) ok = issue_scores(i + 2);
     }
   } else {
-    // ------------------------------------------------------------------ softmax + epilogue: thread = query row
+    // ------------------------------------------------------------------ softmax + epilogue: two threads per query row
     const int q4 = warp & 3, r = q4 * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(q4 * 32) << 16;
     const bool live = r < R;
     const int qpos = live ? first_pos + r : -1;
     const float sc2 = a.scale * 1.4426950408889634f;
-    float m_ref = -INFINITY, l = 0.f;
+    float m_ref = -INFINITY, l = 0.f, alpha = 1.f;
     bool ok = true;
+    // the maximum of a row over both halves of tile i -> reference maximum and factor of what came before
+    auto row_max = [&](int i, float mx) -> bool {
+      float* x = xchg + (i & 1) * 256;
+      x[hf * 128 + r] = mx;
+      mbar_arrive(&x_bar[q4]);
+      if (!mbar_wait_bounded(&x_bar[q4], i & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 0x5000 + i); return false; }
+      mx = fmaxf(x[r], x[128 + r]);
+      alpha = 1.f;
+      if (mx > m_ref + 8.f) {
+        if (m_ref != -INFINITY) { alpha = exp2f(m_ref - mx); l *= alpha; }
+        m_ref = mx;
+      }
+      return true;
+    };
     for (int i = 0; i < n_tiles; ++i) {
       if (!mbar_wait_bounded(&s_full[i & 1], (i >> 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, i); ok = false; break; }
       tc_fence_after();
-      const uint32_t s_addr = tmem + lane_addr + ((i & 1) ? S1_COL : S0_COL);
+      const uint32_t s_addr = tmem + lane_addr + ((i & 1) ? S1_COL : S0_COL) + hf * 64;
       const int key0 = i * PF_KT;
       const bool all_visible = key0 + PF_KT - 1 <= first_pos;      // CTA-uniform: every key of the tile is visible to every live row
       // two passes over the tile's 128 score columns: row maximum, then exponentials packed to bf16 pairs (64 registers).
       // Tiles below the diagonal need no mask (CTA-uniform test), which is all but the last one or two of a long context.
       float mx = -INFINITY;
-      uint32_t pk[PF_KT / 2];
+      uint32_t pk[PF_KT / 4];
       float psum = 0.f;
-      float alpha = 1.f;
       if (all_visible) {           // CTA-uniform (the tensor-memory loads below are warp collectives); rows past R hold zero queries
 #pragma unroll 1
-        for (int c = 0; c < PF_KT / 32; ++c) {
+        for (int c = 0; c < PF_KT / 64; ++c) {
           uint32_t sr[32];
           tmem_ld_x16(s_addr + c * 32, sr);
           tmem_ld_x16(s_addr + c * 32 + 16, sr + 16);
@@ -244,19 +267,16 @@ __global__ void __launch_bounds__(192, 1) mla_prefill_kernel(const __grid_consta
           for (int j = 0; j < 32; ++j) mx = fmaxf(mx, __uint_as_float(sr[j]));
         }
         mx *= sc2;                                   // sc2 > 0: scaling commutes with the maximum
-        if (mx > m_ref + 8.f) {
-          if (m_ref != -INFINITY) { alpha = exp2f(m_ref - mx); l *= alpha; }
-          m_ref = mx;
-        }
+        if (!row_max(i, mx)) { ok = false; break; }
 #pragma unroll
-        for (int c = 0; c < PF_KT / 32; ++c) {
+        for (int c = 0; c < PF_KT / 64; ++c) {
           uint32_t sr[32];
           tmem_ld_x16(s_addr + c * 32, sr);
           tmem_ld_x16(s_addr + c * 32 + 16, sr + 16);
           tc_wait_ld();
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            const float e0 = exp2f(fmaf(__uint_as_float(sr[2 * j]), sc2, -m_ref)), e1 = exp2f(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -m_ref));
+            const float e0 = pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -m_ref)), e1 = pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -m_ref));
             psum += e0 + e1;
             bf162 h = __floats2bfloat162_rn(e0, e1);
             pk[c * 16 + j] = *(uint32_t*)&h;
@@ -264,32 +284,29 @@ __global__ void __launch_bounds__(192, 1) mla_prefill_kernel(const __grid_consta
         }
       } else {
 #pragma unroll 1
-        for (int c = 0; c < PF_KT / 32; ++c) {
+        for (int c = 0; c < PF_KT / 64; ++c) {
           uint32_t sr[32];
           tmem_ld_x16(s_addr + c * 32, sr);
           tmem_ld_x16(s_addr + c * 32 + 16, sr + 16);
           tc_wait_ld();
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            const int kp = key0 + c * 32 + j;
+            const int kp = key0 + hf * 64 + c * 32 + j;
             if (live && kp <= qpos) mx = fmaxf(mx, __uint_as_float(sr[j]) * sc2);
           }
         }
-        if (mx > m_ref + 8.f) {
-          if (m_ref != -INFINITY) { alpha = exp2f(m_ref - mx); l *= alpha; }
-          m_ref = mx;
-        }
+        if (!row_max(i, mx)) { ok = false; break; }
 #pragma unroll
-        for (int c = 0; c < PF_KT / 32; ++c) {
+        for (int c = 0; c < PF_KT / 64; ++c) {
           uint32_t sr[32];
           tmem_ld_x16(s_addr + c * 32, sr);
           tmem_ld_x16(s_addr + c * 32 + 16, sr + 16);
           tc_wait_ld();
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            const int kp = key0 + c * 32 + 2 * j;
-            const float e0 = (live && kp <= qpos) ? exp2f(fmaf(__uint_as_float(sr[2 * j]), sc2, -m_ref)) : 0.f;
-            const float e1 = (live && kp + 1 <= qpos) ? exp2f(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -m_ref)) : 0.f;
+            const int kp = key0 + hf * 64 + c * 32 + 2 * j;
+            const float e0 = (live && kp <= qpos) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -m_ref)) : 0.f;
+            const float e1 = (live && kp + 1 <= qpos) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -m_ref)) : 0.f;
             psum += e0 + e1;
             bf162 h = __floats2bfloat162_rn(e0, e1);
             pk[c * 16 + j] = *(uint32_t*)&h;
@@ -304,7 +321,7 @@ __global__ void __launch_bounds__(192, 1) mla_prefill_kernel(const __grid_consta
       tc_fence_after();
       if (i > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {      // warp-uniform: tcgen05.ld/st are warp collectives
 #pragma unroll 1
-        for (int c = 0; c < NV * 4; ++c) {
+        for (int c = hf * NV * 2; c < (hf + 1) * NV * 2; ++c) {
           uint32_t o[16];
           tmem_ld_x16(tmem + lane_addr + O_COL + c * 16, o);
           tc_wait_ld();
@@ -314,16 +331,20 @@ __global__ void __launch_bounds__(192, 1) mla_prefill_kernel(const __grid_consta
         }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       }
-      // P: two K-major chunks of 64 keys; 16-byte unit u of a row holds keys 8 u .. 8 u + 7
+      // P: two K-major chunks of 64 keys, one per half; 16-byte unit u of a row holds keys 8 u .. 8 u + 7
 #pragma unroll
-      for (int u = 0; u < PF_KT / 8; ++u)
-        *(uint4*)(sP + (u >> 3) * 16384 + r * 128 + (((u & 7) ^ (r & 7)) << 4)) = make_uint4(pk[4 * u], pk[4 * u + 1], pk[4 * u + 2], pk[4 * u + 3]);
+      for (int u = 0; u < PF_KT / 16; ++u)
+        *(uint4*)(sP + hf * 16384 + r * 128 + ((u ^ (r & 7)) << 4)) = make_uint4(pk[4 * u], pk[4 * u + 1], pk[4 * u + 2], pk[4 * u + 3]);
       fence_proxy_async_smem();
       tc_fence_before();
       mbar_arrive(&p_full);
     }
     if (ok && n_tiles > 0 && !mbar_wait_bounded(&o_done, (n_tiles - 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 999); ok = false; }
     tc_fence_after();
+    xchg[(n_tiles & 1) * 256 + hf * 128 + r] = l;                  // the row's sum is that of both halves
+    mbar_arrive(&x_bar[q4]);
+    if (ok && !mbar_wait_bounded(&x_bar[q4], n_tiles & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 998); ok = false; }
+    l = xchg[(n_tiles & 1) * 256 + r] + xchg[(n_tiles & 1) * 256 + 128 + r];
     if (__all_sync(0xffffffffu, ok)) {
       const int t = row_base + (live ? r : 0);
       float scale_o = 1.f, lt = l;
@@ -336,7 +357,7 @@ __global__ void __launch_bounds__(192, 1) mla_prefill_kernel(const __grid_consta
       bf16* dst = a.out + (size_t)t * a.ldo + (size_t)head * a.dv;
       const bool vec = (a.ldo | a.dv) % 8 == 0;
 #pragma unroll 1
-      for (int c = 0; c < NV * 4; ++c) {
+      for (int c = hf * NV * 2; c < (hf + 1) * NV * 2; ++c) {
         uint32_t o[16];
         if (n_tiles > 0) { tmem_ld_x16(tmem + lane_addr + O_COL + c * 16, o); tc_wait_ld(); }
         else {
@@ -374,7 +395,7 @@ template <int KC, int VC>
 struct GqaPrefillCfg {
   static constexpr int K_STAGE = KC * 16384, V_STAGE = VC * 16384;          // chunks (64 dims each) x [128 keys x 128 B]
   static constexpr int NSV = PF_P_BYTES + PF_NS * K_STAGE + 2 * V_STAGE <= 224 * 1024 ? 2 : 1;
-  static constexpr int SMEM = PF_P_BYTES + PF_NS * K_STAGE + NSV * V_STAGE + 256;
+  static constexpr int SMEM = PF_P_BYTES + PF_NS * K_STAGE + NSV * V_STAGE + PF_TAIL;
   static_assert(256 + KC * 32 + VC * 64 <= 512, "scores, query and output exceed tensor memory");
 };
 struct GqaPrefillArgs {
@@ -390,7 +411,7 @@ struct GqaPrefillArgs {
 };
 
 template <int KC, int VC>
-__global__ void __launch_bounds__(192, 1) gqa_prefill_kernel(const __grid_constant__ GqaPrefillArgs a) {
+__global__ void __launch_bounds__(PF_THREADS, 1) gqa_prefill_kernel(const __grid_constant__ GqaPrefillArgs a) {
   using Cf = GqaPrefillCfg<KC, VC>;
   pdl_launch(); pdl_wait();
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -404,8 +425,11 @@ __global__ void __launch_bounds__(192, 1) gqa_prefill_kernel(const __grid_consta
   uint64_t& p_full = bars[12]; uint64_t& o_done = bars[13];
   uint32_t& tmem_slot = *(uint32_t*)(bars + 14);
   int& abort_flag = *(int*)(bars + 15);
+  uint64_t* x_bar = bars + 16;          // [4]: the two softmax warps of a lane quarter
+  float* xchg = (float*)(bars + 32);    // [2][2][128]
   if (smem_u32(smem) & 1023) { if (threadIdx.x == 0) ca_dev_fail(a.status, CA_DEV_BAD_INDEX, 0xA14); return; }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+  const int hf = (warp - 2) >> 2;       // softmax warps: which half of a tile's score columns (and of the output columns)
 
   // the heaviest query tiles (most visible keys) are scheduled first
   const int G = a.Hq / a.Hkv, tok_per_tile = 128 / G;
@@ -429,8 +453,9 @@ __global__ void __launch_bounds__(192, 1) gqa_prefill_kernel(const __grid_consta
 
   if (tid == 0) {
     for (int s = 0; s < 2; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
-    for (int s = 0; s < 2; ++s) { mbar_init(&s_full[s], 1); mbar_init(&s_free[s], 128); }
-    mbar_init(&p_full, 128); mbar_init(&o_done, 1);
+    for (int s = 0; s < 2; ++s) { mbar_init(&s_full[s], 1); mbar_init(&s_free[s], 256); }
+    for (int s = 0; s < 4; ++s) mbar_init(&x_bar[s], 64);
+    mbar_init(&p_full, 256); mbar_init(&o_done, 1);
     abort_flag = 0;
     fence_barrier_init();
   }
@@ -448,7 +473,7 @@ __global__ void __launch_bounds__(192, 1) gqa_prefill_kernel(const __grid_consta
     const int rr = r < R ? r : 0;
     const bf16* src = a.q + (size_t)(row_base + rr / G) * a.q_stride + (size_t)(kvh * G + rr % G) * (KC * 64);
 #pragma unroll 1
-    for (int g = 0; g < KC * 2; ++g) {                  // 16 columns = 32 elements per store
+    for (int g = hf * KC; g < (hf + 1) * KC; ++g) {                  // 16 columns = 32 elements per store
       uint32_t w[16];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -563,7 +588,7 @@ __global__ void __launch_bounds__(192, 1) gqa_prefill_kernel(const __grid_consta
       if (i + 2 < n_tiles) ok = issue_scores(i + 2);
     }
   } else {
-    // ------------------------------------------------------------------ softmax + epilogue: thread = query row
+    // ------------------------------------------------------------------ softmax + epilogue: two threads per query row
     const int q4 = warp & 3, r = q4 * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(q4 * 32) << 16;
     const bool live = r < R;
@@ -571,12 +596,26 @@ __global__ void __launch_bounds__(192, 1) gqa_prefill_kernel(const __grid_consta
     const int wlo = a.window > 0 ? qpos - a.window : -1;           // keys at or below this position are outside the row's window
     const int blocks = live ? a.x.blocks_seen(qpos, a.window) : 0;
     const float sc2 = a.scale * 1.4426950408889634f;
-    float m_ref = -INFINITY, l = 0.f;
+    float m_ref = -INFINITY, l = 0.f, alpha = 1.f;
     bool ok = true;
+    // the maximum of a row over both halves of tile i -> reference maximum and factor of what came before
+    auto row_max = [&](int i, float mx) -> bool {
+      float* x = xchg + (i & 1) * 256;
+      x[hf * 128 + r] = mx;
+      mbar_arrive(&x_bar[q4]);
+      if (!mbar_wait_bounded(&x_bar[q4], i & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 0x5000 + i); return false; }
+      mx = fmaxf(x[r], x[128 + r]);
+      alpha = 1.f;
+      if (mx > m_ref + 8.f) {
+        if (m_ref != -INFINITY) { alpha = exp2f(m_ref - mx); l *= alpha; }
+        m_ref = mx;
+      }
+      return true;
+    };
     for (int i = 0; i < n_tiles; ++i) {
       if (!mbar_wait_bounded(&s_full[i & 1], (i >> 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, i); ok = false; break; }
       tc_fence_after();
-      const uint32_t s_addr = tmem + lane_addr + ((i & 1) ? S1_COL : S0_COL);
+      const uint32_t s_addr = tmem + lane_addr + ((i & 1) ? S1_COL : S0_COL) + hf * 64;
       const int key0 = tile_at(i) * PF_KT;
       // CTA-uniform: every key of the tile is visible to every live row (below the diagonal and inside every row's window)
       // (tiles of pooled blocks: of the blocks that a row sees)
@@ -587,12 +626,11 @@ __global__ void __launch_bounds__(192, 1) gqa_prefill_kernel(const __grid_consta
       // two passes over the tile's 128 score columns: row maximum, then exponentials packed to bf16 pairs (64 registers).
       // Tiles below the diagonal need no mask (CTA-uniform test), which is all but the last one or two of a long context.
       float mx = -INFINITY;
-      uint32_t pk[PF_KT / 2];
+      uint32_t pk[PF_KT / 4];
       float psum = 0.f;
-      float alpha = 1.f;
       if (all_visible) {           // CTA-uniform (the tensor-memory loads below are warp collectives); rows past R hold zero queries
 #pragma unroll 1
-        for (int c = 0; c < PF_KT / 32; ++c) {
+        for (int c = 0; c < PF_KT / 64; ++c) {
           uint32_t sr[32];
           tmem_ld_x16(s_addr + c * 32, sr);
           tmem_ld_x16(s_addr + c * 32 + 16, sr + 16);
@@ -601,19 +639,16 @@ __global__ void __launch_bounds__(192, 1) gqa_prefill_kernel(const __grid_consta
           for (int j = 0; j < 32; ++j) mx = fmaxf(mx, __uint_as_float(sr[j]));
         }
         mx *= sc2;                                   // sc2 > 0: scaling commutes with the maximum
-        if (mx > m_ref + 8.f) {
-          if (m_ref != -INFINITY) { alpha = exp2f(m_ref - mx); l *= alpha; }
-          m_ref = mx;
-        }
+        if (!row_max(i, mx)) { ok = false; break; }
 #pragma unroll
-        for (int c = 0; c < PF_KT / 32; ++c) {
+        for (int c = 0; c < PF_KT / 64; ++c) {
           uint32_t sr[32];
           tmem_ld_x16(s_addr + c * 32, sr);
           tmem_ld_x16(s_addr + c * 32 + 16, sr + 16);
           tc_wait_ld();
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            const float e0 = exp2f(fmaf(__uint_as_float(sr[2 * j]), sc2, -m_ref)), e1 = exp2f(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -m_ref));
+            const float e0 = pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -m_ref)), e1 = pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -m_ref));
             psum += e0 + e1;
             bf162 h = __floats2bfloat162_rn(e0, e1);
             pk[c * 16 + j] = *(uint32_t*)&h;
@@ -621,32 +656,29 @@ __global__ void __launch_bounds__(192, 1) gqa_prefill_kernel(const __grid_consta
         }
       } else {
 #pragma unroll 1
-        for (int c = 0; c < PF_KT / 32; ++c) {
+        for (int c = 0; c < PF_KT / 64; ++c) {
           uint32_t sr[32];
           tmem_ld_x16(s_addr + c * 32, sr);
           tmem_ld_x16(s_addr + c * 32 + 16, sr + 16);
           tc_wait_ld();
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            const int kp = key0 + c * 32 + j;
+            const int kp = key0 + hf * 64 + c * 32 + j;
             if (sees(kp)) mx = fmaxf(mx, __uint_as_float(sr[j]) * sc2);
           }
         }
-        if (mx > m_ref + 8.f) {
-          if (m_ref != -INFINITY) { alpha = exp2f(m_ref - mx); l *= alpha; }
-          m_ref = mx;
-        }
+        if (!row_max(i, mx)) { ok = false; break; }
 #pragma unroll
-        for (int c = 0; c < PF_KT / 32; ++c) {
+        for (int c = 0; c < PF_KT / 64; ++c) {
           uint32_t sr[32];
           tmem_ld_x16(s_addr + c * 32, sr);
           tmem_ld_x16(s_addr + c * 32 + 16, sr + 16);
           tc_wait_ld();
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            const int kp = key0 + c * 32 + 2 * j;
-            const float e0 = sees(kp) ? exp2f(fmaf(__uint_as_float(sr[2 * j]), sc2, -m_ref)) : 0.f;
-            const float e1 = sees(kp + 1) ? exp2f(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -m_ref)) : 0.f;
+            const int kp = key0 + hf * 64 + c * 32 + 2 * j;
+            const float e0 = sees(kp) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -m_ref)) : 0.f;
+            const float e1 = sees(kp + 1) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -m_ref)) : 0.f;
             psum += e0 + e1;
             bf162 h = __floats2bfloat162_rn(e0, e1);
             pk[c * 16 + j] = *(uint32_t*)&h;
@@ -661,7 +693,7 @@ __global__ void __launch_bounds__(192, 1) gqa_prefill_kernel(const __grid_consta
       tc_fence_after();
       if (i > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {      // warp-uniform: tcgen05.ld/st are warp collectives
 #pragma unroll 1
-        for (int c = 0; c < VC * 4; ++c) {
+        for (int c = hf * VC * 2; c < (hf + 1) * VC * 2; ++c) {
           uint32_t o[16];
           tmem_ld_x16(tmem + lane_addr + O_COL + c * 16, o);
           tc_wait_ld();
@@ -671,16 +703,20 @@ __global__ void __launch_bounds__(192, 1) gqa_prefill_kernel(const __grid_consta
         }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       }
-      // P: two K-major chunks of 64 keys; 16-byte unit u of a row holds keys 8 u .. 8 u + 7
+      // P: two K-major chunks of 64 keys, one per half; 16-byte unit u of a row holds keys 8 u .. 8 u + 7
 #pragma unroll
-      for (int u = 0; u < PF_KT / 8; ++u)
-        *(uint4*)(sP + (u >> 3) * 16384 + r * 128 + (((u & 7) ^ (r & 7)) << 4)) = make_uint4(pk[4 * u], pk[4 * u + 1], pk[4 * u + 2], pk[4 * u + 3]);
+      for (int u = 0; u < PF_KT / 16; ++u)
+        *(uint4*)(sP + hf * 16384 + r * 128 + ((u ^ (r & 7)) << 4)) = make_uint4(pk[4 * u], pk[4 * u + 1], pk[4 * u + 2], pk[4 * u + 3]);
       fence_proxy_async_smem();
       tc_fence_before();
       mbar_arrive(&p_full);
     }
     if (ok && n_tiles > 0 && !mbar_wait_bounded(&o_done, (n_tiles - 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 999); ok = false; }
     tc_fence_after();
+    xchg[(n_tiles & 1) * 256 + hf * 128 + r] = l;                  // the row's sum is that of both halves
+    mbar_arrive(&x_bar[q4]);
+    if (ok && !mbar_wait_bounded(&x_bar[q4], n_tiles & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 998); ok = false; }
+    l = xchg[(n_tiles & 1) * 256 + r] + xchg[(n_tiles & 1) * 256 + 128 + r];
     if (__all_sync(0xffffffffu, ok)) {
       const int rr = live ? r : 0;
       const int t = row_base + rr / G, h = kvh * G + rr % G;
@@ -696,7 +732,7 @@ __global__ void __launch_bounds__(192, 1) gqa_prefill_kernel(const __grid_consta
       bf16* dst = a.out + (size_t)t * a.ldo + (size_t)h * a.dv;
       const bool vec = ((a.dv | a.ldo) & 7) == 0;
 #pragma unroll 1
-      for (int c = 0; c < VC * 4; ++c) {
+      for (int c = hf * VC * 2; c < (hf + 1) * VC * 2; ++c) {
         uint32_t o[16];
         if (n_tiles > 0) { tmem_ld_x16(tmem + lane_addr + O_COL + c * 16, o); tc_wait_ld(); }
         else {
@@ -739,7 +775,7 @@ static int launch_gqa_prefill(const GqaPrefillArgs& a, int n_seq, cudaStream_t s
     if (e != cudaSuccess) return ca_cuda(e, "cudaFuncSetAttribute(gqa_prefill)");
     attr_set[dev & 63] = true;
   }
-  CA_LAUNCH_PDL((gqa_prefill_kernel<KC, VC>), dim3(a.Hkv, n_seq * a.max_q_tiles), 192, smem, s, a);
+  CA_LAUNCH_PDL((gqa_prefill_kernel<KC, VC>), dim3(a.Hkv, n_seq * a.max_q_tiles), PF_THREADS, smem, s, a);
   CA_CHECK_LAUNCH("gqa_prefill_attention");
   return CA_OK;
 }
@@ -823,7 +859,7 @@ extern "C" int cuteafd_latent_gather_ctx(const void* cache, const int* page_tabl
 
 template <int KN, int KR, int NV>
 static int mla_prefill_launch(const MlaPrefillArgs& a, int n_seq, cudaStream_t s) {
-  constexpr int SMEM = PF_P_BYTES + PF_NS * (KN + KR) * 16384 + PF_NSV * NV * 16384 + 256;
+  constexpr int SMEM = PF_P_BYTES + PF_NS * (KN + KR) * 16384 + PF_NSV * NV * 16384 + PF_TAIL;
   auto kern = mla_prefill_kernel<KN, KR, NV>;
   static bool attr_set[64] = {false};
   int dev = 0; cudaGetDevice(&dev);
@@ -832,7 +868,7 @@ static int mla_prefill_launch(const MlaPrefillArgs& a, int n_seq, cudaStream_t s
     if (e != cudaSuccess) return ca_cuda(e, "cudaFuncSetAttribute(mla_prefill)");
     attr_set[dev & 63] = true;
   }
-  CA_LAUNCH_PDL(kern, dim3(a.Hl, n_seq * a.max_q_tiles), 192, SMEM, s, a);
+  CA_LAUNCH_PDL(kern, dim3(a.Hl, n_seq * a.max_q_tiles), PF_THREADS, SMEM, s, a);
   return CA_OK;
 }
 
