@@ -1064,13 +1064,13 @@ extern "C" int cuteafd_tc_linear(int kind, int swiglu, int tn, const void* tmA, 
 #endif
     }
   }
-  // 128-row token tiles take the wide kernel where its units (128 tokens x 256 weight rows) occupy a quarter of the SMs: 4096 bf16 rows x 12288 x
-  // 2048 take 160 us there and 420 here, 300 NVFP4 rows x 9216 x 4096 18 and 36, 1024 bf16 rows x 2048 x 4096 (32 units) 26 and 31.  Below that
-  // the narrow kernel's split of K is the better use of the machine.
+  // 128-row token tiles take the wide kernel from an eighth of the SMs' units (128 tokens x 256 weight rows) on: 4096 bf16 rows x 12288 x 2048 take
+  // 160 us there and 420 here, 130 NVFP4 rows x 4096 x 8192 (32 units) 26 and 30, 2331 bf16 rows x 128 x 4096 (19 units) 24 and 26; below, a chain of
+  // stages is the same length in both and this kernel's tiles are narrower (1024 rows x 256 x 7168, 8 units: 45 and 41).
   if (tn == 128 && max_ctas <= 0 && a.splits == 1 && kind != KIND_W4A8 && !peer.n && !grp_rows && act < 2 && !a.trace &&
       (kind == KIND_BF16 || (ldsfb % 16 == 0 && ((uintptr_t)sfb & 15) == 0) || (kind == KIND_MXFP4 && ldsfb % 8 == 0 && ((uintptr_t)sfb & 7) == 0))) {
     const long long items = tiles ? max_tiles : (rows_total + 127) / 128, units = items * (swiglu ? n_nt : (N + 255) / 256);
-    if (4 * units >= ca_sm_count()) {
+    if (8 * units >= ca_sm_count()) {
       WideArgs wa = {};
       wa.tmX = a.tmB; wa.tmW = a.tmA; wa.tmW2 = a.tmA2; wa.sfw = a.sfa; wa.sfw2 = a.sfa2; wa.sfx = a.sfb; wa.ldsfx = ldsfb; wa.alpha = alpha; wa.alpha2 = alpha2;
       wa.tiles = a.tiles; wa.n_tiles = n_tiles; wa.Y = Y; wa.R = a.R; wa.status = status; wa.q_out = a.q_out; wa.sf_out = a.sf_out; wa.inv_gs_out = inv_gs_out;

@@ -355,12 +355,27 @@ class Engine:
                 if tiles * s <= self.sm_count and nkb // s >= 2 and (kind == KIND_FP8B or kind not in CLUSTER_KINDS or tiles <= ops.cluster_capacity(kind, tn, s)):
                     return s
             return 1
-        # larger token tiles: global-memory fix-up (measured on B200: its cost grows with the split count, the sweet
+        if tn >= 128:
+            # prompt-sized tiles: the fix-up through global memory costs more than the idle SMs (4096 rows, bf16 128 x 4096: 48 us in four parts, 25 whole;
+            # 130 rows, NVFP4 4096 x 8192: 57 in two, 26 whole)
+            return 1
+        # tiles of 64 rows: global-memory fix-up (measured on B200: its cost grows with the split count, the sweet
         # spot is about one work unit per SM and never more than 8 splits)
         return max(1, min(nkb // 2, 8, self.sm_count // tiles))
 
+    def _tiling(self, w, x_act, T: int) -> tuple:
+        """(operand, split of K) of a dense product.  Steps of 17 to 64 rows, bf16: tiles of 32 rows where a cluster can split K between them in one
+        wave (32 rows x 2048 x 4096: 10 us, against 21 with 64-row tiles and the fix-up through global memory), else 64-row tiles in one piece
+        (12288 x 2048: 15 us, 17 with narrow ones); FP8 always narrow tiles (two CTAs per SM: 1536 x 7168 11 and 29, 24576 x 1536 11 and 42)."""
+        if x_act.tn == 64 and 16 < T <= 64 and w.kind in (KIND_BF16, KIND_FP8B):
+            splits = self._splits(w.N, w.K, T, 32, w.kind)
+            if splits > 1 or w.kind == KIND_FP8B:
+                return x_act.retiled(32), splits
+            return x_act, 1
+        return x_act, self._splits(w.N, w.K, T, x_act.tn, w.kind)
+
     def _dense(self, w, x_act, y, T, residual=None, w_up=None):
-        splits = 1 if w_up is not None else self._splits(w.N, w.K, T, x_act.tn, w.kind)
+        x_act, splits = (x_act, 1) if w_up is not None else self._tiling(w, x_act, T)
         ops.tc_linear(w, x_act, y, rows=T, w_up=w_up, residual=residual, splits=splits, status=self.status)
         self.launches_per_step += 1
 

@@ -261,6 +261,15 @@ class ActBuffer:
         sf = torch.zeros(rows, -(-K // 256) * (256 // vec), dtype=torch.uint8, device=device)   # padded to whole stages
         return ActBuffer(kind, rows, K, tn, data, encode_tmap(data, tn), sf)
 
+    def retiled(self, tn: int) -> "ActBuffer":
+        """The same rows in token tiles of `tn` (made once, in the eager run of a new shape)."""
+        if tn == self.tn:
+            return self
+        made = self.__dict__.setdefault("_retiled", {})
+        if tn not in made:
+            made[tn] = ActBuffer(self.kind, self.rows, self.K, tn, self.data, encode_tmap(self.data, tn), self.sf)
+        return made[tn]
+
     @staticmethod
     def wrap_bf16(x: torch.Tensor, tn: int) -> "ActBuffer":
         _chk(x, torch.bfloat16, "x")
