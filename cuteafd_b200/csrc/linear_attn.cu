@@ -1,4 +1,4 @@
-// Gated delta-rule linear attention (the recurrent layers of the GDN / KDA hybrid families): decode, verify and short prefill runs.
+// Gated delta-rule linear attention (the recurrent layers of the GDN / KDA hybrid families): decode, verify and prompt runs.
 //
 // Per (sequence, head) a state S [dk x dv] in fp32 is carried from token to token:
 //     S   <- diag(g_t) S                       g_t: decay, one scalar per head (GDN) or one value per key channel (KDA), in (0, 1]
