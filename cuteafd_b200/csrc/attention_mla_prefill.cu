@@ -18,7 +18,7 @@
 // run the softmax, two threads per row, each in two passes over half of the tile's 128 score columns (maximum, which the two exchange
 // through shared memory, then exponentials, which are computed BEFORE the wait for the PV product of tile i - 1, so that product runs
 // under them).  With one thread per row a tile's softmax was a single warp's chain per scheduler and bounded the loop:
-// 2048 rows over 8192 keys of 128 heads 1600 us, 1360 now; 4096 rows of 64 heads over 4 (the paged form below) 834 and 608.
+// 2048 rows over 8192 keys of 128 heads 1600 us, 1430 now; 4096 rows of 64 heads over 4 (the paged form below) 830 and 635.
 // Every wait is bounded and reports through the status word.
 //
 // Reference: the dedicated MLA prefill kernels of the GLM5 family (native/families/glm5/cuda/glm_mla_prefill.cu:123, 539),
@@ -34,7 +34,7 @@
 #define PF_NSV 2                  // V stages
 #define PF_Q_BYTES 0              // the query tile lives in tensor memory (A operand of the score MMAs)
 #define PF_THREADS 320            // producer, MMA issuer, 2 x 4 softmax warps
-#define PF_TAIL 2304              // barriers (256 bytes), row maxima of the two halves of a tile (2 x 2 x 128 floats)
+#define PF_TAIL 2304              // barriers (256 bytes), what the two threads of a row exchange (2 x 2 x 128 floats)
 #define PF_P_BYTES 32768          // 2 chunks (64 keys each) x [128 rows x 128 B]
 #define PF_V_STAGE 32768          // 2 chunks (64 dims each) x [128 keys x 128 B]
 
@@ -68,6 +68,61 @@ __device__ __forceinline__ uint64_t pf_desc_mn_sw128(uint32_t saddr, uint32_t lb
 }
 // 2^x; results below 2^-126 are 0 (exp2f spends three more instructions on them)
 __device__ __forceinline__ float pf_exp2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+// The softmax of a query row that two threads share, thread `hf` with columns 64 hf .. 64 hf + 63 of every 128-key tile.  The row's sum is taken key after
+// key, tile after tile, as one thread would: half 0 sums its pairs of a tile as they come, half 1 holds its own 32 and adds them behind half 0's
+// sum under the next tile's exponentials, so only half 1 knows `l`.  A layer's router and quantisers look at these bits: with a sum per half, added at
+// the end, a latent prompt of 327 tokens chose other experts and its logits moved by 0.05.  The order costs 4 % (1383 and 611 us without it).
+// `xchg` [2][2][128] floats: the halves' maxima of tile i in buffer i & 1; half 0's sum of tile i - 1 travels in half 1's slot of the other buffer,
+// which half 0 has read by then and half 1 writes again only after it read the sum.  `bar` counts both warps' lanes, one phase per tile.
+struct PfRow {
+  float m_ref = -INFINITY, l = 0.f, alpha = 1.f, run = 0.f;
+  float held[PF_KT / 4];
+  float* x; uint64_t* bar;
+  int hf, r;
+  __device__ __forceinline__ PfRow(float* xchg, uint64_t* bar_, int hf_, int r_) : x(xchg), bar(bar_), hf(hf_), r(r_) {
+#pragma unroll
+    for (int j = 0; j < PF_KT / 4; ++j) held[j] = 0.f;
+  }
+  // Phase i of the exchange; afterwards `run` is where this thread's additions start.
+  __device__ __forceinline__ bool meet(int i, volatile int* abortp) {
+    if (hf == 0) x[((i + 1) & 1) * 256 + 128 + r] = run;
+    mbar_arrive(bar);
+    if (!mbar_wait_bounded(bar, i & 1, abortp)) return false;
+    run = hf ? x[((i + 1) & 1) * 256 + 128 + r] : 0.f;
+    return true;
+  }
+  // this half's maximum of tile i -> reference maximum of the row and factor of what came before
+  __device__ __forceinline__ bool row_max(int i, float mx, volatile int* abortp) {
+    float* xi = x + (i & 1) * 256;
+    xi[hf * 128 + r] = mx;
+    if (!meet(i, abortp)) return false;
+    mx = fmaxf(mx, xi[(hf ^ 1) * 128 + r]);
+    alpha = 1.f;
+    if (mx > m_ref + 8.f) {
+      if (m_ref != -INFINITY) alpha = exp2f(m_ref - mx);
+      m_ref = mx;
+    }
+    return true;
+  }
+  // pair j of this thread's columns of the tile
+  __device__ __forceinline__ void add(int j, float pair) { run += hf ? held[j] : pair; held[j] = pair; }
+  // behind a tile's pairs: half 1 has the sum of the tile before
+  __device__ __forceinline__ void next() { l = (l + run) * alpha; }
+  // both threads leave with the row's sum
+  __device__ __forceinline__ bool finish(int n_tiles, volatile int* abortp) {
+    if (!meet(n_tiles, abortp)) return false;
+    if (hf) {
+#pragma unroll
+      for (int j = 0; j < PF_KT / 4; ++j) run += held[j];
+      l += run;
+      x[(n_tiles & 1) * 256 + 128 + r] = l;
+    }
+    mbar_arrive(bar);
+    if (!mbar_wait_bounded(bar, (n_tiles + 1) & 1, abortp)) return false;
+    l = x[(n_tiles & 1) * 256 + 128 + r];
+    return true;
+  }
+};
 __device__ __forceinline__ uint32_t pf_idesc(int n, int b_mn_major) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)b_mn_major << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
@@ -229,22 +284,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) mla_prefill_kernel(const __grid
     const bool live = r < R;
     const int qpos = live ? first_pos + r : -1;
     const float sc2 = a.scale * 1.4426950408889634f;
-    float m_ref = -INFINITY, l = 0.f, alpha = 1.f;
+    PfRow row(xchg, &x_bar[q4], hf, r);
     bool ok = true;
-    // the maximum of a row over both halves of tile i -> reference maximum and factor of what came before
-    auto row_max = [&](int i, float mx) -> bool {
-      float* x = xchg + (i & 1) * 256;
-      x[hf * 128 + r] = mx;
-      mbar_arrive(&x_bar[q4]);
-      if (!mbar_wait_bounded(&x_bar[q4], i & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 0x5000 + i); return false; }
-      mx = fmaxf(x[r], x[128 + r]);
-      alpha = 1.f;
-      if (mx > m_ref + 8.f) {
-        if (m_ref != -INFINITY) { alpha = exp2f(m_ref - mx); l *= alpha; }
-        m_ref = mx;
-      }
-      return true;
-    };
     for (int i = 0; i < n_tiles; ++i) {
       if (!mbar_wait_bounded(&s_full[i & 1], (i >> 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, i); ok = false; break; }
       tc_fence_after();
@@ -255,7 +296,6 @@ __global__ void __launch_bounds__(PF_THREADS, 1) mla_prefill_kernel(const __grid
       // Tiles below the diagonal need no mask (CTA-uniform test), which is all but the last one or two of a long context.
       float mx = -INFINITY;
       uint32_t pk[PF_KT / 4];
-      float psum = 0.f;
       if (all_visible) {           // CTA-uniform (the tensor-memory loads below are warp collectives); rows past R hold zero queries
 #pragma unroll 1
         for (int c = 0; c < PF_KT / 64; ++c) {
@@ -267,7 +307,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) mla_prefill_kernel(const __grid
           for (int j = 0; j < 32; ++j) mx = fmaxf(mx, __uint_as_float(sr[j]));
         }
         mx *= sc2;                                   // sc2 > 0: scaling commutes with the maximum
-        if (!row_max(i, mx)) { ok = false; break; }
+        if (!row.row_max(i, mx, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 0x5000 + i); ok = false; break; }
 #pragma unroll
         for (int c = 0; c < PF_KT / 64; ++c) {
           uint32_t sr[32];
@@ -276,8 +316,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) mla_prefill_kernel(const __grid
           tc_wait_ld();
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            const float e0 = pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -m_ref)), e1 = pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -m_ref));
-            psum += e0 + e1;
+            const float e0 = pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -row.m_ref)), e1 = pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -row.m_ref));
+            row.add(c * 16 + j, e0 + e1);
             bf162 h = __floats2bfloat162_rn(e0, e1);
             pk[c * 16 + j] = *(uint32_t*)&h;
           }
@@ -295,7 +335,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) mla_prefill_kernel(const __grid
             if (live && kp <= qpos) mx = fmaxf(mx, __uint_as_float(sr[j]) * sc2);
           }
         }
-        if (!row_max(i, mx)) { ok = false; break; }
+        if (!row.row_max(i, mx, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 0x5000 + i); ok = false; break; }
 #pragma unroll
         for (int c = 0; c < PF_KT / 64; ++c) {
           uint32_t sr[32];
@@ -305,28 +345,28 @@ __global__ void __launch_bounds__(PF_THREADS, 1) mla_prefill_kernel(const __grid
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int kp = key0 + hf * 64 + c * 32 + 2 * j;
-            const float e0 = (live && kp <= qpos) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -m_ref)) : 0.f;
-            const float e1 = (live && kp + 1 <= qpos) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -m_ref)) : 0.f;
-            psum += e0 + e1;
+            const float e0 = (live && kp <= qpos) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -row.m_ref)) : 0.f;
+            const float e1 = (live && kp + 1 <= qpos) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -row.m_ref)) : 0.f;
+            row.add(c * 16 + j, e0 + e1);
             bf162 h = __floats2bfloat162_rn(e0, e1);
             pk[c * 16 + j] = *(uint32_t*)&h;
           }
         }
       }
-      l += psum;
+      row.next();
       tc_fence_before();
       mbar_arrive(&s_free[i & 1]);
       // the previous P V product must have finished before P is overwritten or O rescaled
       if (i > 0 && !mbar_wait_bounded(&o_done, (i - 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 0x1000 + i); ok = false; break; }
       tc_fence_after();
-      if (i > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {      // warp-uniform: tcgen05.ld/st are warp collectives
+      if (i > 0 && __any_sync(0xffffffffu, row.alpha != 1.f)) {      // warp-uniform: tcgen05.ld/st are warp collectives
 #pragma unroll 1
         for (int c = hf * NV * 2; c < (hf + 1) * NV * 2; ++c) {
           uint32_t o[16];
           tmem_ld_x16(tmem + lane_addr + O_COL + c * 16, o);
           tc_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
+          for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * row.alpha);
           pf_tmem_st_x16(tmem + lane_addr + O_COL + c * 16, o);
         }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -341,17 +381,14 @@ __global__ void __launch_bounds__(PF_THREADS, 1) mla_prefill_kernel(const __grid
     }
     if (ok && n_tiles > 0 && !mbar_wait_bounded(&o_done, (n_tiles - 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 999); ok = false; }
     tc_fence_after();
-    xchg[(n_tiles & 1) * 256 + hf * 128 + r] = l;                  // the row's sum is that of both halves
-    mbar_arrive(&x_bar[q4]);
-    if (ok && !mbar_wait_bounded(&x_bar[q4], n_tiles & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 998); ok = false; }
-    l = xchg[(n_tiles & 1) * 256 + r] + xchg[(n_tiles & 1) * 256 + 128 + r];
+    if (ok && !row.finish(n_tiles, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 998); ok = false; }
     if (__all_sync(0xffffffffu, ok)) {
       const int t = row_base + (live ? r : 0);
-      float scale_o = 1.f, lt = l;
+      float scale_o = 1.f, lt = row.l;
       if (a.sink) {                                     // learned sink logit: one more softmax term with a zero value
-        const float m_nat = (m_ref == -INFINITY) ? -INFINITY : m_ref * 0.6931471805599453f, sk = a.sink[head], m2 = fmaxf(m_nat, sk);
+        const float m_nat = (row.m_ref == -INFINITY) ? -INFINITY : row.m_ref * 0.6931471805599453f, sk = a.sink[head], m2 = fmaxf(m_nat, sk);
         const float e1 = (m_nat == -INFINITY) ? 0.f : __expf(m_nat - m2);
-        lt = l * e1 + __expf(sk - m2); scale_o = e1;
+        lt = row.l * e1 + __expf(sk - m2); scale_o = e1;
       }
       const float inv = (lt > 0.f ? scale_o / lt : 0.f) * ((a.gate && live) ? a.gate[(size_t)t * a.Hl + head] : 1.f);      // output gate of the head
       bf16* dst = a.out + (size_t)t * a.ldo + (size_t)head * a.dv;
@@ -596,22 +633,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) gqa_prefill_kernel(const __grid
     const int wlo = a.window > 0 ? qpos - a.window : -1;           // keys at or below this position are outside the row's window
     const int blocks = live ? a.x.blocks_seen(qpos, a.window) : 0;
     const float sc2 = a.scale * 1.4426950408889634f;
-    float m_ref = -INFINITY, l = 0.f, alpha = 1.f;
+    PfRow row(xchg, &x_bar[q4], hf, r);
     bool ok = true;
-    // the maximum of a row over both halves of tile i -> reference maximum and factor of what came before
-    auto row_max = [&](int i, float mx) -> bool {
-      float* x = xchg + (i & 1) * 256;
-      x[hf * 128 + r] = mx;
-      mbar_arrive(&x_bar[q4]);
-      if (!mbar_wait_bounded(&x_bar[q4], i & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 0x5000 + i); return false; }
-      mx = fmaxf(x[r], x[128 + r]);
-      alpha = 1.f;
-      if (mx > m_ref + 8.f) {
-        if (m_ref != -INFINITY) { alpha = exp2f(m_ref - mx); l *= alpha; }
-        m_ref = mx;
-      }
-      return true;
-    };
     for (int i = 0; i < n_tiles; ++i) {
       if (!mbar_wait_bounded(&s_full[i & 1], (i >> 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, i); ok = false; break; }
       tc_fence_after();
@@ -627,7 +650,6 @@ __global__ void __launch_bounds__(PF_THREADS, 1) gqa_prefill_kernel(const __grid
       // Tiles below the diagonal need no mask (CTA-uniform test), which is all but the last one or two of a long context.
       float mx = -INFINITY;
       uint32_t pk[PF_KT / 4];
-      float psum = 0.f;
       if (all_visible) {           // CTA-uniform (the tensor-memory loads below are warp collectives); rows past R hold zero queries
 #pragma unroll 1
         for (int c = 0; c < PF_KT / 64; ++c) {
@@ -639,7 +661,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) gqa_prefill_kernel(const __grid
           for (int j = 0; j < 32; ++j) mx = fmaxf(mx, __uint_as_float(sr[j]));
         }
         mx *= sc2;                                   // sc2 > 0: scaling commutes with the maximum
-        if (!row_max(i, mx)) { ok = false; break; }
+        if (!row.row_max(i, mx, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 0x5000 + i); ok = false; break; }
 #pragma unroll
         for (int c = 0; c < PF_KT / 64; ++c) {
           uint32_t sr[32];
@@ -648,8 +670,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) gqa_prefill_kernel(const __grid
           tc_wait_ld();
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            const float e0 = pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -m_ref)), e1 = pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -m_ref));
-            psum += e0 + e1;
+            const float e0 = pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -row.m_ref)), e1 = pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -row.m_ref));
+            row.add(c * 16 + j, e0 + e1);
             bf162 h = __floats2bfloat162_rn(e0, e1);
             pk[c * 16 + j] = *(uint32_t*)&h;
           }
@@ -667,7 +689,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) gqa_prefill_kernel(const __grid
             if (sees(kp)) mx = fmaxf(mx, __uint_as_float(sr[j]) * sc2);
           }
         }
-        if (!row_max(i, mx)) { ok = false; break; }
+        if (!row.row_max(i, mx, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 0x5000 + i); ok = false; break; }
 #pragma unroll
         for (int c = 0; c < PF_KT / 64; ++c) {
           uint32_t sr[32];
@@ -677,28 +699,28 @@ __global__ void __launch_bounds__(PF_THREADS, 1) gqa_prefill_kernel(const __grid
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int kp = key0 + hf * 64 + c * 32 + 2 * j;
-            const float e0 = sees(kp) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -m_ref)) : 0.f;
-            const float e1 = sees(kp + 1) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -m_ref)) : 0.f;
-            psum += e0 + e1;
+            const float e0 = sees(kp) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -row.m_ref)) : 0.f;
+            const float e1 = sees(kp + 1) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -row.m_ref)) : 0.f;
+            row.add(c * 16 + j, e0 + e1);
             bf162 h = __floats2bfloat162_rn(e0, e1);
             pk[c * 16 + j] = *(uint32_t*)&h;
           }
         }
       }
-      l += psum;
+      row.next();
       tc_fence_before();
       mbar_arrive(&s_free[i & 1]);
       // the previous P V product must have finished before P is overwritten or O rescaled
       if (i > 0 && !mbar_wait_bounded(&o_done, (i - 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 0x1000 + i); ok = false; break; }
       tc_fence_after();
-      if (i > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {      // warp-uniform: tcgen05.ld/st are warp collectives
+      if (i > 0 && __any_sync(0xffffffffu, row.alpha != 1.f)) {      // warp-uniform: tcgen05.ld/st are warp collectives
 #pragma unroll 1
         for (int c = hf * VC * 2; c < (hf + 1) * VC * 2; ++c) {
           uint32_t o[16];
           tmem_ld_x16(tmem + lane_addr + O_COL + c * 16, o);
           tc_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
+          for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * row.alpha);
           pf_tmem_st_x16(tmem + lane_addr + O_COL + c * 16, o);
         }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -713,19 +735,16 @@ __global__ void __launch_bounds__(PF_THREADS, 1) gqa_prefill_kernel(const __grid
     }
     if (ok && n_tiles > 0 && !mbar_wait_bounded(&o_done, (n_tiles - 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 999); ok = false; }
     tc_fence_after();
-    xchg[(n_tiles & 1) * 256 + hf * 128 + r] = l;                  // the row's sum is that of both halves
-    mbar_arrive(&x_bar[q4]);
-    if (ok && !mbar_wait_bounded(&x_bar[q4], n_tiles & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 998); ok = false; }
-    l = xchg[(n_tiles & 1) * 256 + r] + xchg[(n_tiles & 1) * 256 + 128 + r];
+    if (ok && !row.finish(n_tiles, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 998); ok = false; }
     if (__all_sync(0xffffffffu, ok)) {
       const int rr = live ? r : 0;
       const int t = row_base + rr / G, h = kvh * G + rr % G;
-      float scale_o = 1.f, lt = l;
+      float scale_o = 1.f, lt = row.l;
       if (a.x.sink) {                                   // learned sink logit: one more softmax term with a zero value
-        const float m_nat = (m_ref == -INFINITY) ? -INFINITY : m_ref * 0.6931471805599453f;
+        const float m_nat = (row.m_ref == -INFINITY) ? -INFINITY : row.m_ref * 0.6931471805599453f;
         const float sk = a.x.sink[h], m2 = fmaxf(m_nat, sk);
         const float e1 = (m_nat == -INFINITY) ? 0.f : __expf(m_nat - m2);
-        lt = l * e1 + __expf(sk - m2); scale_o = e1;
+        lt = row.l * e1 + __expf(sk - m2); scale_o = e1;
       }
       const float inv = (lt > 0.f ? scale_o / lt : 0.f) * a.x.head_factor(t, h);
       const bool gated = a.x.gate && a.x.gate_values;
