@@ -330,8 +330,8 @@ class Engine:
         self.launches_per_step += 1
 
     # ------------------------------------------------------------------ kernels
-    def _splits(self, N: int, K: int, T: int, tn: int, kind: int) -> int:
-        """Split-K factor of a dense layer.  Decode-sized token tiles (<= 32 rows) split over a thread-block cluster
+    def _splits(self, N: int, K: int, T: int, tn: int, kind: int, f32: bool = False) -> int:
+        """Split-K factor of a dense layer (`f32`: its result is not rounded to bf16).  Decode-sized token tiles (<= 32 rows) split over a thread-block cluster
         (up to 8 CTAs reduce through distributed shared memory): the largest split that still fits one wave - asked of the
         device, since a cluster must sit inside one GPC - and leaves every CTA at least two pipeline stages of K."""
         tiles = -(-N // 128) * -(-T // tn)
@@ -355,15 +355,18 @@ class Engine:
                 if tiles * s <= self.sm_count and nkb // s >= 2 and (kind == KIND_FP8B or kind not in CLUSTER_KINDS or tiles <= ops.cluster_capacity(kind, tn, s)):
                     return s
             return 1
-        if tn >= 128:
-            # prompt-sized tiles: the fix-up through global memory costs more than the idle SMs (4096 rows, bf16 128 x 4096: 48 us in four parts, 25 whole;
-            # 130 rows, NVFP4 4096 x 8192: 57 in two, 26 whole)
+        if tn >= 128 and (kind == KIND_FP8B or (kind == KIND_BF16 and (K <= 2048 or not f32))):
+            # prompt-sized tiles, bf16: the fix-up through global memory costs more than the idle SMs (128-row tiles, 4096 rows x 128 x 2048: 51 us in four parts,
+            # 23 whole; 300 x 2048 x 4096: 59 and 37; 256-row tiles, 300 x 2048 x 4096: 86 and 39).  Long sums that stay fp32 keep their parts: a router
+            # chooses experts by their last bits, and a part rounds less often than one accumulator over all of K (256 x 7168, 4096 rows: 66 us in two
+            # parts, 57 whole).  So do FP4 products (130 rows, 4096 x 8192: 57 and 33), whose results are rounded to four bits next: added in another
+            # order, 150 rows through four layers moved by 0.023, near what their error against 64 bits is.
             return 1
-        # tiles of 64 rows: global-memory fix-up (measured on B200: its cost grows with the split count, the sweet
+        # larger token tiles: global-memory fix-up (measured on B200: its cost grows with the split count, the sweet
         # spot is about one work unit per SM and never more than 8 splits)
         return max(1, min(nkb // 2, 8, self.sm_count // tiles))
 
-    def _tiling(self, w, x_act, T: int) -> tuple:
+    def _tiling(self, w, x_act, T: int, f32: bool = False) -> tuple:
         """(operand, split of K) of a dense product.  Steps of 17 to 64 rows, bf16: tiles of 32 rows where a cluster can split K between them in one
         wave (32 rows x 2048 x 4096: 10 us, against 21 with 64-row tiles and the fix-up through global memory), else 64-row tiles in one piece
         (12288 x 2048: 15 us, 17 with narrow ones); FP8 always narrow tiles (two CTAs per SM: 1536 x 7168 11 and 29, 24576 x 1536 11 and 42)."""
@@ -372,10 +375,10 @@ class Engine:
             if splits > 1 or w.kind == KIND_FP8B:
                 return x_act.retiled(32), splits
             return x_act, 1
-        return x_act, self._splits(w.N, w.K, T, x_act.tn, w.kind)
+        return x_act, self._splits(w.N, w.K, T, x_act.tn, w.kind, f32)
 
     def _dense(self, w, x_act, y, T, residual=None, w_up=None):
-        x_act, splits = (x_act, 1) if w_up is not None else self._tiling(w, x_act, T)
+        x_act, splits = (x_act, 1) if w_up is not None else self._tiling(w, x_act, T, y.dtype == torch.float32)
         ops.tc_linear(w, x_act, y, rows=T, w_up=w_up, residual=residual, splits=splits, status=self.status)
         self.launches_per_step += 1
 

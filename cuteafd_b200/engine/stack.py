@@ -155,14 +155,14 @@ class StackBase:
             x_act = self.lane(T).retiled(x_act, tn)
         super()._dense(w, x_act, y, T, residual=residual, w_up=w_up)
 
-    def _tiling(self, w, x_act, T):
-        return x_act, self._splits(w.N, w.K, T, x_act.tn, w.kind)          # `_dense` chose the tiles
+    def _tiling(self, w, x_act, T, f32=False):
+        return x_act, self._splits(w.N, w.K, T, x_act.tn, w.kind, f32)          # `_dense` chose the tiles
 
-    def _splits(self, N, K, T, tn, kind):
+    def _splits(self, N, K, T, tn, kind, f32=False):
         """Short tiles of 64 rows gain from the fix-up of a split only while they leave three of four SMs idle (measured on B200)."""
         if kind == KIND_F32 or (kind == KIND_BF16 and tn == 64 and T <= 64 and K <= 8192 and 4 * -(-N // 128) > self.sm_count):
             return 1
-        return super()._splits(N, K, T, tn, kind)
+        return super()._splits(N, K, T, tn, kind, f32)
 
     def _experts(self, m, lw, L: StackLane, e: dict, T: int):
         """Routing, packing, gather and the experts' products of the rows L.xn, from router logits in e["logits"]: weighted rows stay in e."""
