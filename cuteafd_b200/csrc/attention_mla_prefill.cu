@@ -18,7 +18,7 @@
 // run the softmax, two threads per row, each in two passes over half of the tile's 128 score columns (maximum, which the two exchange
 // through shared memory, then exponentials, which are computed BEFORE the wait for the PV product of tile i - 1, so that product runs
 // under them).  With one thread per row a tile's softmax was a single warp's chain per scheduler and bounded the loop:
-// 2048 rows over 8192 keys of 128 heads 1600 us, 1430 now; 4096 rows of 64 heads over 4 (the paged form below) 830 and 635.
+// 2048 rows over 8192 keys of 128 heads 1600 us, 1430 now; 4096 rows of 64 heads over 4 (the paged form below) 830 and 640.
 // Every wait is bounded and reports through the status word.
 //
 // Reference: the dedicated MLA prefill kernels of the GLM5 family (native/families/glm5/cuda/glm_mla_prefill.cu:123, 539),
@@ -87,7 +87,7 @@ struct PfRow {
   __device__ __forceinline__ bool meet(int i, volatile int* abortp) {
     if (hf == 0) x[((i + 1) & 1) * 256 + 128 + r] = run;
     mbar_arrive(bar);
-    if (!mbar_wait_bounded(bar, i & 1, abortp)) return false;
+    if (!mbar_wait_warp(bar, i & 1, abortp)) return false;
     run = hf ? x[((i + 1) & 1) * 256 + 128 + r] : 0.f;
     return true;
   }
@@ -118,7 +118,7 @@ struct PfRow {
       x[(n_tiles & 1) * 256 + 128 + r] = l;
     }
     mbar_arrive(bar);
-    if (!mbar_wait_bounded(bar, (n_tiles + 1) & 1, abortp)) return false;
+    if (!mbar_wait_warp(bar, (n_tiles + 1) & 1, abortp)) return false;
     l = x[(n_tiles & 1) * 256 + 128 + r];
     return true;
   }
@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) mla_prefill_kernel(const __grid
     PfRow row(xchg, &x_bar[q4], hf, r);
     bool ok = true;
     for (int i = 0; i < n_tiles; ++i) {
-      if (!mbar_wait_bounded(&s_full[i & 1], (i >> 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, i); ok = false; break; }
+      if (!mbar_wait_warp(&s_full[i & 1], (i >> 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, i); ok = false; break; }
       tc_fence_after();
       const uint32_t s_addr = tmem + lane_addr + ((i & 1) ? S1_COL : S0_COL) + hf * 64;
       const int key0 = i * PF_KT;
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) mla_prefill_kernel(const __grid
       tc_fence_before();
       mbar_arrive(&s_free[i & 1]);
       // the previous P V product must have finished before P is overwritten or O rescaled
-      if (i > 0 && !mbar_wait_bounded(&o_done, (i - 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 0x1000 + i); ok = false; break; }
+      if (i > 0 && !mbar_wait_warp(&o_done, (i - 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 0x1000 + i); ok = false; break; }
       tc_fence_after();
       if (i > 0 && __any_sync(0xffffffffu, row.alpha != 1.f)) {      // warp-uniform: tcgen05.ld/st are warp collectives
 #pragma unroll 1
@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) mla_prefill_kernel(const __grid
       tc_fence_before();
       mbar_arrive(&p_full);
     }
-    if (ok && n_tiles > 0 && !mbar_wait_bounded(&o_done, (n_tiles - 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 999); ok = false; }
+    if (ok && n_tiles > 0 && !mbar_wait_warp(&o_done, (n_tiles - 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 999); ok = false; }
     tc_fence_after();
     if (ok && !row.finish(n_tiles, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 998); ok = false; }
     if (__all_sync(0xffffffffu, ok)) {
@@ -636,7 +636,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) gqa_prefill_kernel(const __grid
     PfRow row(xchg, &x_bar[q4], hf, r);
     bool ok = true;
     for (int i = 0; i < n_tiles; ++i) {
-      if (!mbar_wait_bounded(&s_full[i & 1], (i >> 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, i); ok = false; break; }
+      if (!mbar_wait_warp(&s_full[i & 1], (i >> 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, i); ok = false; break; }
       tc_fence_after();
       const uint32_t s_addr = tmem + lane_addr + ((i & 1) ? S1_COL : S0_COL) + hf * 64;
       const int key0 = tile_at(i) * PF_KT;
@@ -711,7 +711,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) gqa_prefill_kernel(const __grid
       tc_fence_before();
       mbar_arrive(&s_free[i & 1]);
       // the previous P V product must have finished before P is overwritten or O rescaled
-      if (i > 0 && !mbar_wait_bounded(&o_done, (i - 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 0x1000 + i); ok = false; break; }
+      if (i > 0 && !mbar_wait_warp(&o_done, (i - 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 0x1000 + i); ok = false; break; }
       tc_fence_after();
       if (i > 0 && __any_sync(0xffffffffu, row.alpha != 1.f)) {      // warp-uniform: tcgen05.ld/st are warp collectives
 #pragma unroll 1
@@ -733,7 +733,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) gqa_prefill_kernel(const __grid
       tc_fence_before();
       mbar_arrive(&p_full);
     }
-    if (ok && n_tiles > 0 && !mbar_wait_bounded(&o_done, (n_tiles - 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 999); ok = false; }
+    if (ok && n_tiles > 0 && !mbar_wait_warp(&o_done, (n_tiles - 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 999); ok = false; }
     tc_fence_after();
     if (ok && !row.finish(n_tiles, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, 998); ok = false; }
     if (__all_sync(0xffffffffu, ok)) {

@@ -265,6 +265,11 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     if (clock64() - t0 > limit) { *abort_flag = 1; return false; }
   }
 }
+// The same for a whole, converged warp: true only if every lane's wait came through.  Lanes must not give up one by one in front of warp collectives
+// (`tcgen05.ld`, `tcgen05.st`, shuffles): the others would wait in them for good.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag));
+}
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
