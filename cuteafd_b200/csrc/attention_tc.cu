@@ -16,8 +16,10 @@
 // and `attn_merge_kernel` (attention.cu) combines them.
 //
 // Steps of so many sequences that none is split, without a window, cut every sequence by ITS length (`plan_slot`): the launch has a fixed number of
-// slots, each block works out from the lengths which sequence and which part of it its slot is.  48 sequences of 100 to 9,900 tokens (64 query heads over 4):
-// one block each per head, 306 us, as long as the longest; now 150 us.
+// slots, each block works out from the lengths which sequence and which part of it its slot is.  Whole sequences write their rows as ever; the
+// pieces of a cut one leave partials, and the piece that finishes last merges them (no further launch).  48 sequences of 100 to 9,900 tokens (64 query
+// heads over 4): one block each per head, 318 us, as long as the longest; now 156.  48 of 5,000: 174 and 175 us, 48 of 100: 20.5 and 20.6; 40 to 400:
+// 28.8 and 30.7.  (With partials and a merge launch for every sequence: 165, 185, 30 and 40.)
 //
 // Replaces the reference's sparse/GQA attention programs (AOT-exported, sources absent) and its wmma/mma.sync
 // kernels (native/shared/cuda/draft_attention.cu:41-340, families/glm5/cuda/glm_mla_prefill.cu:123-960).
@@ -47,7 +49,7 @@ struct AttnTcArgs {
   int* status;
   int q_stride, Hq, Hkv, max_pages, n_splits, window, max_q_tiles, T;
   int slots, n_seq, wave, max_q; // slots > 0: parts by length; blocks per head and query tile that run at once; longest query run
-  int4* slot_of_row;            // ... and what the merge needs: {first slot, number of slots, row within its sequence} of every query row
+  uint32_t* arrived;            // ... and pieces of a sequence that are done, [n_seq, Hkv, max_q_tiles], zero between launches
   int v_head0, dv, ldo;         // value width of the output (at most VC * 64) and its row pitch: head h at column h * dv
   float scale;
 };
@@ -75,8 +77,10 @@ __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sy
 
 // What slot `slot` of a step holds.  Sequences of uneven length are cut into pieces of about L pages, so many that all pieces fit the slots
 // (sum ceil(p / L) <= n_seq + sum p / L); even ones are left whole (a wave of pieces plus a piece's start-up must be shorter than the longest
-// sequence).  All pieces of a sequence share the reference maximum of its first page (each looks at that page once more), so probabilities are
-// rounded alike however a sequence is cut and only the order of fp32 sums depends on it.  Every lane of the warp must call it.
+// sequence).  All pieces of a sequence start from the reference maximum of its first page (each looks at that page once more): while no score
+// exceeds it by more than 8 binary orders, probabilities are rounded alike however a sequence is cut and only the order of fp32 sums depends on it.
+// Beyond that a piece goes on from a reference of its own, as an uncut sequence does from there on.  So the last bits of a long sequence in an uneven
+// step depend on its neighbours' lengths.  Every lane of the warp must call it.
 struct SlotPlan { int seq, piece, cuts; };               // sequence (-1: the slot is not used), piece of it, its number of pieces
 __device__ __forceinline__ SlotPlan plan_slot(const AttnTcArgs& a, int slot) {
   const int lane = threadIdx.x & 31;
@@ -140,14 +144,14 @@ __global__ void __launch_bounds__(192, AttnTcCfg<KC, VC>::OCC) paged_attn_tc_ker
 
   const int G = a.Hq / a.Hkv;
   const int tok_per_tile = 128 / G;
-  const int kvh = blockIdx.y;
+  const int kvh = a.slots ? blockIdx.x : blockIdx.y, slot = blockIdx.y;       // slots: those without a piece are the last to start
   int split = blockIdx.x, n_splits = a.n_splits, seq = blockIdx.z / a.max_q_tiles, qt = blockIdx.z % a.max_q_tiles;
   if (a.slots) {
-    const SlotPlan p = plan_slot(a, blockIdx.x);
+    const SlotPlan p = plan_slot(a, slot);
     if (p.seq < 0) return;
     seq = p.seq; split = p.piece; n_splits = p.cuts; qt = blockIdx.z;
   }
-  const bool direct = !a.slots && n_splits == 1;        // else partials for the merge
+  const bool direct = n_splits == 1;        // else partials for the merge
   const int qlen = a.q_len[seq], kvlen = a.kv_len[seq];
   const int tok0 = qt * tok_per_tile;
   if (tok0 >= qlen) return;
@@ -170,7 +174,6 @@ __global__ void __launch_bounds__(192, AttnTcCfg<KC, VC>::OCC) paged_attn_tc_ker
 
   // Decode-shaped tiles (<= 32 real rows) replicate the rows into every 32-lane quarter of the MMA tile so that
   // the four softmax warps each take 16 of the 64 score columns of the SAME rows (4x shorter per-tile chain).
-  if (a.slots && split == 0 && kvh == 0 && tid < ntok) a.slot_of_row[row_base + tid] = make_int4((int)blockIdx.x, n_splits, tok0 + tid, 0);
   const bool rep4 = R <= 32;
   const int n_live_warps = rep4 ? 4 : (R + 31) / 32;    // softmax warps with work
   if (tid == 0) {
@@ -443,7 +446,7 @@ __global__ void __launch_bounds__(192, AttnTcCfg<KC, VC>::OCC) paged_attn_tc_ker
       const bool gated = a.x.gate && a.x.gate_values;
       bf16* dst = a.out + (size_t)t * a.ldo + (size_t)h * a.dv;
       const bool vec = ((a.dv | a.ldo) & 7) == 0;      // otherwise heads do not start on 16 bytes
-      const size_t prow = (a.slots ? (size_t)blockIdx.x * a.max_q + (tok0 + rr / G) : (size_t)split * a.T + t) * a.Hq + h;
+      const size_t prow = (a.slots ? (size_t)slot * a.max_q + (tok0 + rr / G) : (size_t)split * a.T + t) * a.Hq + h;
       float* po = direct ? nullptr : a.part_o + prow * (VC * 64);
 #pragma unroll 1
       for (int c = 0; c < VC * 4; ++c) {
@@ -483,9 +486,28 @@ __global__ void __launch_bounds__(192, AttnTcCfg<KC, VC>::OCC) paged_attn_tc_ker
     }
   }
   if (*abortp && warp == 0) { const uint64_t t0 = globaltimer_ns(); while (globaltimer_ns() - t0 < 200000) __nanosleep(1000); }
+  const bool cut = a.slots && !direct;
+  if (cut) __threadfence();                             // this piece's partials, before it counts as done
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem, Cf::TMEM_COLS);
+  if (cut) {
+    // every piece counts once, also one that gave up, so the counters are zero again behind the launch
+    int& last = *(int*)(bars + 15);
+    if (tid == 0) last = atomicInc(a.arrived + ((size_t)seq * a.Hkv + kvh) * a.max_q_tiles + qt, n_splits - 1) == n_splits - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    constexpr int D = VC * 64;
+    const size_t first = (size_t)slot - split;
+    for (int u = tid; u < R * (D / 8); u += 192) {
+      const int r = u / (D / 8), d0 = (u % (D / 8)) * 8, t = row_base + r / G, h = kvh * G + r % G;
+      float o[8], L;
+      attn_merge8<true>(a.part_o, a.part_ml, a.x.sink != nullptr, a.x.sink ? a.x.sink[h] : -INFINITY, (first * a.max_q + tok0 + r / G) * a.Hq + h, (size_t)a.max_q * a.Hq, n_splits, D, d0, o, L);
+      bf16 ob[8];
+      attn_store8(a.x, a.out, t, h, d0, a.dv, a.ldo, o, L, ob);
+    }
+  }
 }
 
 static AttnExtras<bf16> sink_only(const float* sink) {
@@ -506,7 +528,7 @@ static int launch_attn_tc(const AttnTcArgs& a, int n_seq, cudaStream_t s) {
   }
   // No pre-fill of the (m, l) partials: every CTA writes them for all of its live rows, also when its split
   // holds no key (m = -inf, l = 0), and a CTA that gives up reports through the status word.
-  CA_LAUNCH_PDL((paged_attn_tc_kernel<KC, VC>), a.slots ? dim3(a.slots, a.Hkv, a.max_q_tiles) : dim3(a.n_splits, a.Hkv, n_seq * a.max_q_tiles), 192, smem, s, a);
+  CA_LAUNCH_PDL((paged_attn_tc_kernel<KC, VC>), a.slots ? dim3(a.Hkv, a.slots, a.max_q_tiles) : dim3(a.n_splits, a.Hkv, n_seq * a.max_q_tiles), 192, smem, s, a);
   CA_CHECK_LAUNCH("paged_attention_tc");
   return CA_OK;
 }
@@ -526,7 +548,7 @@ extern "C" int cuteafd_attn_merge(const float* part_o, const float* part_ml, con
   CA_REQUIRE(part_o && part_ml && out && n_parts >= 1, "attn_merge: needs partials");
   if (T <= 0) return CA_OK;
   CA_LAUNCH_PDL(attn_merge8_kernel, dim3(T, (Hq * AD / 8 + 127) / 128), 128, 0, s, part_o, part_ml, sink_only(sink), (bf16*)out, T, Hq, (int)AD, (int)AD, Hq * AD, n_parts,
-                (uint8_t*)nullptr, (uint8_t*)nullptr, 0, (const float*)nullptr, 0, (const int4*)nullptr, 0);
+                (uint8_t*)nullptr, (uint8_t*)nullptr, 0, (const float*)nullptr, 0);
   CA_CHECK_LAUNCH("attn_merge");
   return CA_OK;
 }
@@ -556,7 +578,7 @@ extern "C" int cuteafd_paged_attention_tc(const void* q, const void* kv_map, con
   if (rc != CA_OK) return rc;
   if (n_splits > 1 && !partials_only) {
     CA_LAUNCH_PDL(attn_merge8_kernel, dim3(T, (Hq * AD / 8 + 127) / 128), 128, 0, s, part_o, part_ml, sink_only(sink), (bf16*)out, T, Hq, (int)AD, (int)AD, Hq * AD, n_splits,
-                  (uint8_t*)q_out, (uint8_t*)sf_out, ldsf, inv_gs, qkind, (const int4*)nullptr, 0);
+                  (uint8_t*)q_out, (uint8_t*)sf_out, ldsf, inv_gs, qkind);
     CA_CHECK_LAUNCH("attn_merge");
   }
   return CA_OK;
@@ -564,22 +586,21 @@ extern "C" int cuteafd_paged_attention_tc(const void* q, const void* kv_map, con
 
 // Slots of a step of `n_seq` sequences for the form below: one per sequence, and a wave and a half of blocks for further pieces.  Returns 0 where
 // it does not apply: a step that is split evenly fills a wave already (16 sequences of 4,096 in 4 parts: the plan and the unused slots cost 5 us of
-// 45), and one sequence is always even.
+// 45), and one whose whole sequences leave SMs without a block is not split only because its contexts are a page long.
 extern "C" int cuteafd_attn_slots(int n_seq, int max_q_len, int Hq, int Hkv, int n_splits) {
   if (n_seq < 2 || n_splits != 1 || max_q_len < 1 || max_q_len > 16 || Hkv < 1 || Hq % Hkv || 128 % (Hq / Hkv)) return 0;
   const int tpt = 128 / (Hq / Hkv), tiles = (max_q_len + tpt - 1) / tpt;
+  if ((long long)n_seq * Hkv * tiles <= ca_sm_count()) return 0;
   const int wave = 2 * ca_sm_count() / (Hkv * tiles) > 1 ? 2 * ca_sm_count() / (Hkv * tiles) : 1;
   return n_seq + wave + wave / 2 + 1;
 }
 
 // The same attention (no window) with every sequence split by its length.  part_o / part_ml hold `slots` (cuteafd_attn_slots) x max_q_len rows of Hq
-// partials, slot_of_row int4 [T].
+// partials; `arrived` uint32 [n_seq * Hq] (at least a counter per sequence, KV head and query tile), zero before the first launch, is left zero.
 extern "C" int cuteafd_paged_attention_slots(const void* q, const void* kv_map, const int* page_table, const int* kv_len, const int* q_start, const int* q_len,
-                                             const float* sink, void* out, float* part_o, float* part_ml, void* slot_of_row, int T, int n_seq, int max_q_len, int q_stride,
-                                             int Hq, int Hkv, int max_pages, int slots, float scale, int* status, void* q_out, void* sf_out, int ldsf,
-                                             const float* inv_gs, int qkind, cudaStream_t s) {
-  CA_REQUIRE(qkind == 0 || (q_out && sf_out && (Hq * AD) % 256 == 0), "paged_attention_slots: FP4 output needs buffers and Hq*128 %% 256 == 0");
-  CA_REQUIRE(part_o && part_ml && slot_of_row && ((uintptr_t)slot_of_row & 15) == 0, "paged_attention_slots: needs scratch");
+                                             const float* sink, void* out, float* part_o, float* part_ml, void* arrived, int T, int n_seq, int max_q_len, int q_stride,
+                                             int Hq, int Hkv, int max_pages, int slots, float scale, int* status, cudaStream_t s) {
+  CA_REQUIRE(part_o && part_ml && arrived && (((uintptr_t)part_o | (uintptr_t)part_ml) & 15) == 0, "paged_attention_slots: needs scratch");
   CA_REQUIRE(slots > 0 && slots == cuteafd_attn_slots(n_seq, max_q_len, Hq, Hkv, 1), "paged_attention_slots: %d slots", slots);
   CA_REQUIRE(q_stride % 8 == 0, "paged_attention_slots: q rows must be 16-byte aligned");
   if (T <= 0) return CA_OK;
@@ -589,14 +610,9 @@ extern "C" int cuteafd_paged_attention_slots(const void* q, const void* kv_map, 
   a.q_stride = q_stride; a.Hq = Hq; a.Hkv = Hkv; a.max_pages = max_pages; a.n_splits = 1; a.T = T; a.scale = scale;
   const int tpt = 128 / (Hq / Hkv);
   a.max_q_tiles = (max_q_len + tpt - 1) / tpt;
-  a.slots = slots; a.n_seq = n_seq; a.max_q = max_q_len; a.slot_of_row = (int4*)slot_of_row;
+  a.slots = slots; a.n_seq = n_seq; a.max_q = max_q_len; a.arrived = (uint32_t*)arrived;
   a.wave = 2 * ca_sm_count() / (Hkv * a.max_q_tiles) > 1 ? 2 * ca_sm_count() / (Hkv * a.max_q_tiles) : 1;
-  const int rc = launch_attn_tc<2, 2>(a, n_seq, s);
-  if (rc != CA_OK) return rc;
-  CA_LAUNCH_PDL(attn_merge8_kernel, dim3(T, (Hq * AD / 8 + 127) / 128), 128, 0, s, part_o, part_ml, sink_only(sink), (bf16*)out, T, Hq, (int)AD, (int)AD, Hq * AD, 1,
-                (uint8_t*)q_out, (uint8_t*)sf_out, ldsf, inv_gs, qkind, (const int4*)slot_of_row, max_q_len);
-  CA_CHECK_LAUNCH("attn_merge");
-  return CA_OK;
+  return launch_attn_tc<2, 2>(a, n_seq, s);
 }
 
 // Descriptor for one layer's paged K/V store [slots, 2, Hkv, 128] bf16: dims {128, 2*Hkv, slots}, box {64, 1, 64}.
@@ -638,7 +654,7 @@ extern "C" int cuteafd_window_attention(const void* q, const void* maps, const i
   if (rc != CA_OK) return rc;
   if (n_splits > 1) {
     CA_LAUNCH_PDL(attn_merge8_kernel, dim3(T, (Hq * dv_pad / 8 + 127) / 128), 128, 0, s, part_o, part_ml, a.x, (bf16*)out, T, Hq, dv_pad, dv, ldo, n_splits,
-                  (uint8_t*)nullptr, (uint8_t*)nullptr, 0, (const float*)nullptr, 0, (const int4*)nullptr, 0);
+                  (uint8_t*)nullptr, (uint8_t*)nullptr, 0, (const float*)nullptr, 0);
     CA_CHECK_LAUNCH("attn_merge");
   }
   return CA_OK;

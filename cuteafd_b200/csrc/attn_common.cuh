@@ -27,40 +27,33 @@ static __global__ void attn_merge_kernel(const float* __restrict__ part_o, const
   }
 }
 
-// Same merge, eight output elements per thread (the first Dout of a head's D columns, head h at column h * Dout of rows ldo apart), optionally also writing the merged row quantised to FP4 for the
-// output projection that follows (qkind 1 NVFP4 / 2 MXFP4; needs Hq * D % 256 == 0).  grid (T, ceil(Hq * D / 8 / 128)).
-static __global__ void attn_merge8_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, const AttnExtras<bf16> x,
-                                          bf16* __restrict__ out, int T, int Hq, int D, int Dout, int ldo, int n_splits, uint8_t* __restrict__ q,
-                                          uint8_t* __restrict__ sf, int ldsf, const float* __restrict__ inv_gs_ptr, int qkind, const int4* __restrict__ slots, int max_q) {
-  // `slots` (null: every row has n_splits partials): {first partial, number of partials, row within its sequence} of every query row, whose
-  // partials lie [partial][max_q][Hq].
-  pdl_launch(); pdl_wait();
-  const int t = blockIdx.x, vi = blockIdx.y * blockDim.x + threadIdx.x, vpr = D / 8;
-  if (vi >= Hq * vpr) return;                     // whole warps leave together (Hq * D / 8 is a multiple of 32 with FP4 output)
-  const int h = vi / vpr, d0 = (vi % vpr) * 8;
-  // Up to eight splits at a time, every load issued before the first use: the (m, l) pairs and the partial rows of all splits are
-  // in flight together (a loop that reads m, branches, then loads the row is one L2 round trip per split on a decode step's
-  // critical path).  Partial rows of empty splits (m = -inf) are loaded but not used; the buffers always cover every split.
-  int first = 0, qrow = t, pitch = T;
-  if (slots) { const int4 m = slots[t]; first = m.x; n_splits = m.y; qrow = m.z; pitch = max_q; }
-  const float sk = x.sink ? x.sink[h] : -INFINITY;
-  float M = sk, L = 0.f;
-  float o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int s0 = 0; s0 < n_splits; s0 += 8) {
+// The merge for eight output elements of one (row, head): partial i lies at row0 + i * step of `part_ml` (pairs) and `part_o` (D columns), its
+// columns from d0 on.  FRESH: other blocks of this kernel have just written them (no read-only cache).  Leaves the unnormalised sum in o and
+// its denominator in L.
+// Up to eight partials at a time, every load issued before the first use: the (m, l) pairs and the partial rows are in flight together (a loop
+// that reads m, branches, then loads the row is one L2 round trip per partial on a decode step's critical path).  Partial rows of empty
+// splits (m = -inf) are loaded but not used; the buffers always cover every split.
+template <bool FRESH>
+__device__ __forceinline__ void attn_merge8(const float* part_o, const float* part_ml, bool sink, float sk, size_t row0, size_t step, int n, int D, int d0, float (&o)[8], float& L) {
+  float M = sk;
+  L = 0.f;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) o[q] = 0.f;
+  for (int s0 = 0; s0 < n; s0 += 8) {
     float2 ml[8]; float4 pa[8], pb[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const int s = min(s0 + j, n_splits - 1);
-      const size_t row = ((size_t)(first + s) * pitch + qrow) * Hq + h;
-      ml[j] = *(const float2*)(part_ml + row * 2);
+      const size_t row = row0 + min(s0 + j, n - 1) * step;
+      const float2* pm = (const float2*)(part_ml + row * 2);
       const float4* po = (const float4*)(part_o + row * D + d0);
-      pa[j] = po[0]; pb[j] = po[1];
+      if (FRESH) { ml[j] = __ldcg(pm); pa[j] = __ldcg(po); pb[j] = __ldcg(po + 1); }
+      else { ml[j] = __ldg(pm); pa[j] = __ldg(po); pb[j] = __ldg(po + 1); }
     }
     float Mn = M;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) if (s0 + j < n_splits) Mn = fmaxf(Mn, ml[j].x);
+    for (int j = 0; j < 8; ++j) if (s0 + j < n) Mn = fmaxf(Mn, ml[j].x);
     if (s0 == 0) {
-      if (x.sink) L = __expf(sk - Mn);                  // the sink's share first, as the one-pass form adds it
+      if (sink) L = __expf(sk - Mn);                    // the sink's share first, as the one-pass form adds it
     } else if (Mn != M && M != -INFINITY) {           // a later batch raised the maximum: rescale what was accumulated
       const float r = __expf(M - Mn);
       L *= r;
@@ -70,7 +63,7 @@ static __global__ void attn_merge8_kernel(const float* __restrict__ part_o, cons
     M = Mn;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      if (s0 + j < n_splits && ml[j].x != -INFINITY) {
+      if (s0 + j < n && ml[j].x != -INFINITY) {
         const float e = __expf(ml[j].x - M);
         L += ml[j].y * e;
         o[0] += pa[j].x * e; o[1] += pa[j].y * e; o[2] += pa[j].z * e; o[3] += pa[j].w * e;
@@ -78,9 +71,11 @@ static __global__ void attn_merge8_kernel(const float* __restrict__ part_o, cons
       }
     }
   }
+}
 
+// Eight merged elements -> bf16 `ob` and the output row (the first Dout of a head's D columns, head h at column h * Dout of rows ldo apart).
+__device__ __forceinline__ void attn_store8(const AttnExtras<bf16>& x, bf16* out, int t, int h, int d0, int Dout, int ldo, float (&o)[8], float L, bf16 (&ob)[8]) {
   const float inv = (L > 0.f ? 1.f / L : 0.f) * x.head_factor(t, h);
-  bf16 ob[8];
   if (x.gate && x.gate_values) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) if (d0 + j < Dout) o[j] *= x.value_factor(t, h * Dout + d0 + j);
@@ -93,6 +88,21 @@ static __global__ void attn_merge8_kernel(const float* __restrict__ part_o, cons
 #pragma unroll
     for (int j = 0; j < 8; ++j) if (d0 + j < Dout) dst[j] = ob[j];
   }
+}
+
+// That merge as a launch, eight output elements per thread, optionally also writing the merged row quantised to FP4 for the
+// output projection that follows (qkind 1 NVFP4 / 2 MXFP4; needs Hq * D % 256 == 0).  grid (T, ceil(Hq * D / 8 / 128)).
+static __global__ void attn_merge8_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, const AttnExtras<bf16> x,
+                                          bf16* __restrict__ out, int T, int Hq, int D, int Dout, int ldo, int n_splits, uint8_t* __restrict__ q,
+                                          uint8_t* __restrict__ sf, int ldsf, const float* __restrict__ inv_gs_ptr, int qkind) {
+  pdl_launch(); pdl_wait();
+  const int t = blockIdx.x, vi = blockIdx.y * blockDim.x + threadIdx.x, vpr = D / 8;
+  if (vi >= Hq * vpr) return;                     // whole warps leave together (Hq * D / 8 is a multiple of 32 with FP4 output)
+  const int h = vi / vpr, d0 = (vi % vpr) * 8;
+  float o[8], L;
+  attn_merge8<false>(part_o, part_ml, x.sink != nullptr, x.sink ? x.sink[h] : -INFINITY, (size_t)t * Hq + h, (size_t)T * Hq, n_splits, D, d0, o, L);
+  bf16 ob[8];
+  attn_store8(x, out, t, h, d0, Dout, ldo, o, L, ob);
   if (qkind) {
     float f[8];
 #pragma unroll

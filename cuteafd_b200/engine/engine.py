@@ -511,10 +511,9 @@ class Engine:
                         ptr(md["q_len"]), ptr(lw.sink), ptr(L.attn), T, sh.n_seq, sh.max_q_len, L.qkv.shape[1], a.n_heads, a.n_kv_heads,
                         md["page_table"].shape[1], window, a.head_dim ** -0.5, ptr(self.status), native.stream())
         elif slots:
-            fused_q = ops.paged_attention_slots(L.qkv, self.kv_tmaps[li], md["page_table"], md["kv_len"], md["q_start"], md["q_len"], L.attn, T=T, n_seq=sh.n_seq,
-                                                max_q_len=sh.max_q_len, q_stride=L.qkv.shape[1], Hq=a.n_heads, Hkv=a.n_kv_heads,
-                                                slots=slots, part_o=self.part_o, part_ml=self.part_ml, slot_of_row=self.part_rows, sink=lw.sink,
-                                                status=self.status, quant=L.attn_q, inv_gs=lw.wo.inv_act_gs)
+            ops.paged_attention_slots(L.qkv, self.kv_tmaps[li], md["page_table"], md["kv_len"], md["q_start"], md["q_len"], L.attn, T=T, n_seq=sh.n_seq,
+                                      max_q_len=sh.max_q_len, q_stride=L.qkv.shape[1], Hq=a.n_heads, Hkv=a.n_kv_heads,
+                                      slots=slots, part_o=self.part_o, part_ml=self.part_ml, arrived=self.part_done, sink=lw.sink, status=self.status)
         elif self.kv_tmaps is not None:
             fused_q = ops.paged_attention_tc(L.qkv, self.kv_tmaps[li], md["page_table"], md["kv_len"], md["q_start"], md["q_len"], L.attn,
                                              T=T, n_seq=sh.n_seq, max_q_len=sh.max_q_len, q_stride=L.qkv.shape[1], Hq=a.n_heads,
@@ -527,7 +526,7 @@ class Engine:
                                 window=window, sink=lw.sink)
         oq = L.attn_q if fused_q else self._quant(L.attn, L.attn_q, T, lw.wo.inv_act_gs)
         self._attn_out(li, lw, oq, L, T)
-        self.launches_per_step += 2 + (1 if sh.attn_splits > 1 or slots else 0)
+        self.launches_per_step += 2 + (1 if sh.attn_splits > 1 else 0)
 
     _ffn_in_quantised = False
     _tokens_quantised = False          # the FFN norm left the experts' operand of every token in the lane's `xt`
@@ -744,9 +743,8 @@ class Engine:
                 self._part_keep = getattr(self, "_part_keep", []) + [(getattr(self, "part_o", None), getattr(self, "part_ml", None))]     # captured steps hold them
                 self.part_o = torch.empty(need * a.head_dim, dtype=torch.float32, device=self.device)
                 self.part_ml = torch.empty(need * 2, dtype=torch.float32, device=self.device)
-            if slots and (getattr(self, "part_rows", None) is None or self.part_rows.shape[0] < T):
-                self._part_keep = getattr(self, "_part_keep", []) + [getattr(self, "part_rows", None)]
-                self.part_rows = torch.zeros(max(T, 256), 4, dtype=torch.int32, device=self.device)
+            if slots and getattr(self, "part_done", None) is None:
+                self.part_done = torch.zeros(self.max_seqs * a.n_heads, dtype=torch.int32, device=self.device)
         elif getattr(self, "part_o", None) is None:
             self.part_o = self.part_ml = None
 

@@ -631,16 +631,12 @@ def attn_slots(n_seq: int, max_q_len: int, Hq: int, Hkv: int, n_splits: int) -> 
     return native.lib().cuteafd_attn_slots(n_seq, max_q_len, Hq, Hkv, n_splits)
 
 
-def paged_attention_slots(q, kv_map, page_table, kv_len, q_start, q_len, out, *, T, n_seq, max_q_len, q_stride, Hq, Hkv, slots, part_o, part_ml, slot_of_row,
-                          sink=None, scale=None, status=None, quant=None, inv_gs=None) -> bool:
-    """`paged_attention_tc` (one split, no window) for steps of at least two sequences of at most 16 rows, every sequence cut by its length.  part_o fp32
-    [slots * max_q_len * Hq * 128], part_ml fp32 [.. * 2], slot_of_row int32 [T, 4].  True: `quant` was written too."""
-    fused = quant is not None and quant.kind in FP4_KINDS and (Hq * 128) % 256 == 0
+def paged_attention_slots(q, kv_map, page_table, kv_len, q_start, q_len, out, *, T, n_seq, max_q_len, q_stride, Hq, Hkv, slots, part_o, part_ml, arrived,
+                          sink=None, scale=None, status=None):
+    """`paged_attention_tc` (one split, no window) with every sequence cut by its length; for steps that `attn_slots` gives slots.  part_o fp32
+    [slots * max_q_len * Hq * 128], part_ml fp32 [.. * 2]; arrived int32 [n_seq * Hq], zero, and left zero."""
     call("cuteafd_paged_attention_slots", ptr(q), ptr(kv_map), ptr(page_table), ptr(kv_len), ptr(q_start), ptr(q_len), ptr(sink), ptr(out), ptr(part_o), ptr(part_ml),
-         ptr(slot_of_row), T, n_seq, max_q_len, q_stride, Hq, Hkv, page_table.shape[1], slots, float(scale if scale is not None else 128 ** -0.5), ptr(status),
-         ptr(quant.data) if fused else None, ptr(quant.sf) if fused else None, quant.sf.shape[1] if fused else 0, ptr(inv_gs) if fused else None,
-         (2 if quant.kind == KIND_MXFP4 else 1) if fused else 0, stream())
-    return fused
+         ptr(arrived), T, n_seq, max_q_len, q_stride, Hq, Hkv, page_table.shape[1], slots, float(scale if scale is not None else 128 ** -0.5), ptr(status), stream())
 
 
 def attn_merge(part_o, part_ml, out, *, T, Hq, n_parts, sink=None):

@@ -52,7 +52,7 @@ _PROTOS = {
     "cuteafd_moe_combine": [P, P, P, P, P, P, I, I, I, P, P],
     "cuteafd_paged_attention": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, F, P],
     "cuteafd_attn_slots": [I, I, I, I, I],
-    "cuteafd_paged_attention_slots": [P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, P, P, P, I, P, I, P],
+    "cuteafd_paged_attention_slots": [P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, P, P],
     "cuteafd_paged_attention_tc": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, P, P, P, I, P, I, P],
     "cuteafd_tmap_encode_kv": [P, P, I, U64],
     "cuteafd_mla_attention": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, F, P, P],
