@@ -728,6 +728,21 @@ class Engine:
             self.launches_per_step += 4
         return L
 
+    def _grown(self, name: str, n: int) -> torch.Tensor:
+        """The fp32 scratch `name`, at least `n` elements.  An outgrown one stays, since captured steps hold its address; each is at least twice the one
+        before, so all of them together are smaller than the one in use."""
+        buf = getattr(self, name, None)
+        if buf is not None and buf.numel() >= n:
+            return buf
+        from ..utils.memory_ledger import LEDGER
+        n = max(n, 2 * buf.numel()) if buf is not None else n
+        with LEDGER.scope("workspace/attention"):
+            LEDGER.charge(4 * n, name)
+        if buf is not None:
+            self.__dict__.setdefault("_outgrown", []).append(buf)
+        setattr(self, name, torch.empty(n, dtype=torch.float32, device=self.device))
+        return getattr(self, name)
+
     def _attn_slots(self, sh: StepShape) -> int:
         """Blocks per head that cut the step's sequences by their lengths (0: every sequence into `attn_splits`)."""
         a = self.spec.attn
@@ -738,11 +753,7 @@ class Engine:
         slots = self._attn_slots(sh)
         rows = max(sh.attn_splits * T if sh.attn_splits > 1 else 0, slots * sh.max_q_len)
         if rows:
-            need = rows * a.n_heads
-            if getattr(self, "part_o", None) is None or self.part_o.numel() < need * a.head_dim:
-                self._part_keep = getattr(self, "_part_keep", []) + [(getattr(self, "part_o", None), getattr(self, "part_ml", None))]     # captured steps hold them
-                self.part_o = torch.empty(need * a.head_dim, dtype=torch.float32, device=self.device)
-                self.part_ml = torch.empty(need * 2, dtype=torch.float32, device=self.device)
+            self.part_o, self.part_ml = self._grown("part_o", rows * a.n_heads * a.head_dim), self._grown("part_ml", rows * a.n_heads * 2)
             if slots and getattr(self, "part_done", None) is None:
                 self.part_done = torch.zeros(self.max_seqs * a.n_heads, dtype=torch.int32, device=self.device)
         elif getattr(self, "part_o", None) is None:
