@@ -274,12 +274,8 @@ class MlaEngine(Engine):
         qn_act = self._act(b, ("qn", T, tn), q_nope, tn)
         ops.tc_linear(w.w_uk_t, qn_act, q_lat, rows=Hl * T, tiles=tiles, n_tiles=n_tiles, max_tiles=max_tiles, status=self.status)
         o_lat = b["o_lat"][:Hl * T]
-        if sh.attn_splits > 1:
-            need = sh.attn_splits * T * Hl
-            if getattr(self, "mla_part_o", None) is None or self.mla_part_o.numel() < need * DV:
-                self.mla_part_o = torch.empty(need * DV, dtype=torch.float32, device=self.device)
-                self.mla_part_ml = torch.empty(need * 2, dtype=torch.float32, device=self.device)
-        po, pml = (self.mla_part_o, self.mla_part_ml) if sh.attn_splits > 1 else (None, None)
+        need = sh.attn_splits * T * Hl
+        po, pml = (self._grown("mla_part_o", need * DV), self._grown("mla_part_ml", need * 2)) if sh.attn_splits > 1 else (None, None)
         scale = (a.qk_nope_head_dim + a.qk_rope_head_dim) ** -0.5
         call("cuteafd_mla_attention", ptr(q_lat), ptr(b["q_rope"]), ptr(self.kv_tmaps[li]), ptr(md["page_table"]), ptr(md["kv_len"]),
              ptr(md["q_start"]), ptr(md["q_len"]), ptr(o_lat), ptr(po), ptr(pml), T, sh.n_seq, sh.max_q_len, Hl, md["page_table"].shape[1],
@@ -361,10 +357,7 @@ class MlaEngine(Engine):
         po = pml = None
         if splits > 1:
             need = splits * T * Hl
-            if getattr(self, "mla_part_o", None) is None or self.mla_part_o.numel() < need * DV:
-                self.mla_part_o = torch.empty(need * DV, dtype=torch.float32, device=dev)
-                self.mla_part_ml = torch.empty(need * 2, dtype=torch.float32, device=dev)
-            po, pml = self.mla_part_o, self.mla_part_ml
+            po, pml = self._grown("mla_part_o", need * DV), self._grown("mla_part_ml", need * 2)
         scale = (a.qk_nope_head_dim + a.qk_rope_head_dim) ** -0.5
         call("cuteafd_mla_attention", ptr(q_lat), ptr(b["q_rope"]), ptr(self._dsa["gmap"]), ptr(st["pages"]), ptr(st["count"]), ptr(st["q_start"]),
              ptr(st["q_len"]), ptr(o_lat), ptr(po), ptr(pml), T, T, 1, Hl, kp // PAGE, splits, scale, sp, stream())

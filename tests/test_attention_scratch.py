@@ -28,3 +28,15 @@ def test_a_growing_batch_outgrows_few_buffers(monkeypatch):
     assert sum(b.numel() for b in seen[:-1]) <= seen[-1].numel() and eng.part_o is seen[-1] and eng.part_done is done and done.numel() == 64 * 64
     held = seen + [eng.part_ml] + [b for b in eng._outgrown if not any(b is k for k in seen)]
     assert LEDGER.by_scope["workspace/attention"] - charged == 4 * sum(b.numel() for b in held)
+
+
+def test_latent_engines_grow_theirs_the_same_way():
+    """A captured step holds the address of the scratch that it was captured with, so nothing that a larger step outgrew is given back."""
+    eng = types.SimpleNamespace(device="cpu")
+    first = Engine._grown(eng, "mla_part_o", 1000)
+    assert Engine._grown(eng, "mla_part_o", 900) is first
+    second = Engine._grown(eng, "mla_part_o", 1001)
+    assert second.numel() == 2000 and eng._outgrown == [first] and eng.mla_part_o is second
+    import inspect
+    from cuteafd_b200.engine import mla
+    assert "self.mla_part_o =" not in inspect.getsource(mla)
