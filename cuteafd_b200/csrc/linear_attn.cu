@@ -275,9 +275,10 @@ extern "C" int cuteafd_gated_delta_run(const void* q, const void* k, const void*
   a.q_start = q_start; a.q_len = q_len; a.out = (bf16*)out; a.snapshots = snapshots; a.H = H; a.per_channel = per_channel; a.n_slots = n_slots;
   a.status = status;
   const dim3 grid(H * (LA_DV / LA_COLS), n_seq);
-  // the four-block form loads four channels at a time
+  // the four-block form loads four channels at a time, and every block all of a head's q and k: no output may take their place
+  const bool in_place = out == q || out == k;
   const bool aligned = (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 7) == 0 && (!(per_channel & 1) || ((uintptr_t)g & 15) == 0);
-  if (!aligned || (max_len > 0 && max_len <= 6 && (long long)H * n_seq * (LA_DV / LA_COLS) > 2 * ca_sm_count())) CA_LAUNCH_PDL(gated_delta_short_kernel, dim3(H, n_seq), LA_DV, 0, s, a);
+  if (!aligned || in_place || (max_len > 0 && max_len <= 6 && (long long)H * n_seq * (LA_DV / LA_COLS) > 2 * ca_sm_count())) CA_LAUNCH_PDL(gated_delta_short_kernel, dim3(H, n_seq), LA_DV, 0, s, a);
   else if (per_channel & 1) { if (snapshots) CA_LAUNCH_PDL((gated_delta_kernel<true, true>), grid, LA_THREADS, 0, s, a); else CA_LAUNCH_PDL((gated_delta_kernel<true, false>), grid, LA_THREADS, 0, s, a); }
   else { if (snapshots) CA_LAUNCH_PDL((gated_delta_kernel<false, true>), grid, LA_THREADS, 0, s, a); else CA_LAUNCH_PDL((gated_delta_kernel<false, false>), grid, LA_THREADS, 0, s, a); }
   CA_CHECK_LAUNCH("gated_delta_step");
@@ -322,8 +323,10 @@ __global__ void __launch_bounds__(128) short_conv4_kernel(const bf16* __restrict
   }
   auto input = [&](int t) { return t >= 0 ? *(const Vec*)(xs + (size_t)t * ldx) : *(const Vec*)(cr + (size_t)(3 + t) * C); };
   // the launch may have fewer token blocks than the longest sequence needs: each takes every gridDim.z-th chunk
+  Vec h0, h1, h2;
   for (int c0 = blockIdx.z * CONV_TOK; c0 < n; c0 += gridDim.z * CONV_TOK) {
-    Vec h0 = input(c0 - 3), h1 = input(c0 - 2), h2 = input(c0 - 1);
+    // (a block that walks the whole sequence has the three inputs in front already, and does not look at rows that it may have written: x == y)
+    if (c0 == 0 || gridDim.z > 1) { h0 = input(c0 - 3); h1 = input(c0 - 2); h2 = input(c0 - 1); }
     Vec in[CONV_TOK];
     const int m = min(CONV_TOK, n - c0);
 #pragma unroll
@@ -354,7 +357,7 @@ static int short_conv4(const void* x, const float* w, void* carry, const int* sl
   if (n_seq <= 0) return CA_OK;
   // a step of few tokens is a chain of latencies: more threads with one channel each
   const bool vec = (max_len <= 0 || max_len > 8) && C % 4 == 0 && ldx % 4 == 0 && (((uintptr_t)x | (uintptr_t)y | (uintptr_t)carry) & 7) == 0;
-  const int V = vec ? 4 : 1, chunks = max_len > 0 ? (max_len + CONV_TOK - 1) / CONV_TOK : 1;
+  const int V = vec ? 4 : 1, chunks = max_len > 0 && x != y ? (max_len + CONV_TOK - 1) / CONV_TOK : 1;      // in place: no block reads what another writes
   const dim3 grid((C + 128 * V - 1) / (128 * V), n_seq, chunks < 1024 ? chunks : 1024);
   if (vec) CA_LAUNCH_PDL((short_conv4_kernel<UPDATE, 4>), grid, 128, 0, s, (const bf16*)x, w, (bf16*)carry, slot_of_seq, q_start, q_len, (bf16*)y, C, ldx, n_slots, status);
   else CA_LAUNCH_PDL((short_conv4_kernel<UPDATE, 1>), grid, 128, 0, s, (const bf16*)x, w, (bf16*)carry, slot_of_seq, q_start, q_len, (bf16*)y, C, ldx, n_slots, status);

@@ -148,3 +148,33 @@ def test_short_conv4_in_token_blocks_matches_reference(C, ldx, lens):
             assert float((y[t0:t0 + n].float().cpu() - want).abs().max()) < 2 ** -7 * float(want.abs().max())
             assert torch.equal(carry[slot].cpu(), b16(after) if update else carry0[slot])
         assert torch.equal(carry[1].cpu(), carry0[1])
+
+
+@pytest.mark.parametrize("lens", [(1, 2, 3), (16, 17, 50), (4, 200, 33)])
+def test_outputs_may_take_the_place_of_inputs(lens):
+    """The convolution over its own rows, and the delta rule's output over its queries, keys or values: as into rows of their own."""
+    g = torch.Generator(device=DEV).manual_seed(sum(lens))
+    H, C, n, T = 4, 384, 3, sum(lens)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    meta, status = [i32(t) for t in ((2, 0, 1), (0, lens[0], lens[0] + lens[1]), lens)], torch.zeros(4, dtype=torch.int32, device=DEV)
+    x, w, carry0 = (torch.randn(*s, generator=g, device=DEV) for s in ((T, C), (C, 4), (n, 3, C)))
+    for max_len in (0, max(lens)):
+        got = []
+        for same in (False, True):
+            rows, carry = x.to(torch.bfloat16), carry0.to(torch.bfloat16)
+            y = rows if same else torch.zeros_like(rows)
+            call("cuteafd_short_conv4_run", ptr(rows), ptr(w), ptr(carry), *map(ptr, meta), ptr(y), n, C, C, n, max_len, 1, ptr(status), stream())
+            got.append((y, carry))
+        torch.cuda.synchronize()
+        assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    unit = lambda: torch.nn.functional.normalize(torch.randn(T, H, 128, generator=g, device=DEV), dim=-1).to(torch.bfloat16)
+    qkv, gate, beta = [unit(), unit(), unit()], torch.rand(T, H, generator=g, device=DEV) * 0.3 + 0.7, torch.rand(T, H, generator=g, device=DEV)
+    for over in (None, 0, 1, 2):
+        args, state = [t.clone() for t in qkv], torch.zeros(n, H, 128, 128, device=DEV)
+        out = torch.zeros_like(qkv[0]) if over is None else args[over]
+        call("cuteafd_gated_delta_run", *map(ptr, args), ptr(gate), ptr(beta), ptr(state), *map(ptr, meta), ptr(out), None, n, H, 0, n, max(lens), ptr(status), stream())
+        torch.cuda.synchronize()
+        want = (out.float(), state) if over is None else want
+        assert float((out.float() - want[0]).abs().max()) <= 2 ** -8 * float(want[0].abs().max())      # a last place of bf16
+        assert torch.allclose(state, want[1], atol=1e-5, rtol=1e-5)
+    assert status.tolist() == [0, 0, 0, 0]
