@@ -262,8 +262,14 @@ __global__ void __launch_bounds__(LA_DV) gated_delta_short_kernel(const LinAttnA
   for (int i = 0; i < LA_DK; ++i) S[(size_t)i * LA_DV + j] = col[i];
 }
 
-// `max_len`: the longest run (0: not known).  Short runs take the short form when the four-block form would need more than one wave (8 sequences x 4
-// tokens x 32 heads: 11 us against 17), and the four-block form otherwise.
+// `max_len`: the longest run (0: not known).  Short runs take the short form when the four-block form would need more than one wave, and the longer
+// the more waves it needs: it has four times the blocks, and a shorter chain per token.  Measured, short / four-block form in us, 32 heads:
+//     sequences     2 tokens       3            4            5            6            7            8
+//       3          12.4 / 14.3  14.5 / 14.5  16.4 / 14.5  18.4 / 16.3  19.5 / 16.4  20.5 / 16.5  22.6 / 14.4        (1.3 waves)
+//       5          14.3 / 16.4  16.4 / 18.3  18.4 / 18.5  18.5 / 18.5  20.7 / 18.8  22.6 / 20.4                     (2.2)
+//       8          14.4 / 20.6  16.4 / 22.5  18.5 / 22.6  20.5 / 24.6  22.6 / 24.6  24.6 / 26.6  26.7 / 24.6        (3.5)
+//      48          51.3 / 79.9  63.5 / 84.0  73.7 / 90.1  84.0 / 94.1  96.3 / 98.3   107 / 103    119 / 94          (21)
+// Not told apart: where the short form itself is just over a wave (5 sequences of 64 heads) its line is at 4 tokens (6 tokens: 34.8 / 28.8).
 extern "C" int cuteafd_gated_delta_run(const void* q, const void* k, const void* v, const float* g, const float* beta, float* state,
                                        const int* slot_of_seq, const int* q_start, const int* q_len, void* out, float* snapshots, int n_seq,
                                        int H, int per_channel, int n_slots, int max_len, int* status, cudaStream_t s) {
@@ -277,8 +283,9 @@ extern "C" int cuteafd_gated_delta_run(const void* q, const void* k, const void*
   const dim3 grid(H * (LA_DV / LA_COLS), n_seq);
   // the four-block form loads four channels at a time, and every block all of a head's q and k: no output may take their place
   const bool in_place = out == q || out == k;
+  const float waves = (float)((long long)H * n_seq * (LA_DV / LA_COLS)) / (float)(2 * ca_sm_count());
   const bool aligned = (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 7) == 0 && (!(per_channel & 1) || ((uintptr_t)g & 15) == 0);
-  if (!aligned || in_place || (max_len > 0 && max_len <= 6 && (long long)H * n_seq * (LA_DV / LA_COLS) > 2 * ca_sm_count())) CA_LAUNCH_PDL(gated_delta_short_kernel, dim3(H, n_seq), LA_DV, 0, s, a);
+  if (!aligned || in_place || (max_len > 0 && waves > 1.f && max_len <= (waves < 3.f ? 2 + (int)waves : 6))) CA_LAUNCH_PDL(gated_delta_short_kernel, dim3(H, n_seq), LA_DV, 0, s, a);
   else if (per_channel & 1) { if (snapshots) CA_LAUNCH_PDL((gated_delta_kernel<true, true>), grid, LA_THREADS, 0, s, a); else CA_LAUNCH_PDL((gated_delta_kernel<true, false>), grid, LA_THREADS, 0, s, a); }
   else { if (snapshots) CA_LAUNCH_PDL((gated_delta_kernel<false, true>), grid, LA_THREADS, 0, s, a); else CA_LAUNCH_PDL((gated_delta_kernel<false, false>), grid, LA_THREADS, 0, s, a); }
   CA_CHECK_LAUNCH("gated_delta_step");

@@ -178,3 +178,24 @@ def test_outputs_may_take_the_place_of_inputs(lens):
         assert float((out.float() - want[0]).abs().max()) <= 2 ** -8 * float(want[0].abs().max())      # a last place of bf16
         assert torch.allclose(state, want[1], atol=1e-5, rtol=1e-5)
     assert status.tolist() == [0, 0, 0, 0]
+
+
+@pytest.mark.parametrize("n,rows", [(9, 3), (10, 3), (10, 4), (19, 4), (19, 5), (28, 6), (28, 7)])
+def test_runs_on_both_sides_of_the_line_between_the_forms(n, rows):
+    """8 heads: one wave and just more, two and three waves, with the longest run that still takes the short form there and one more."""
+    g = torch.Generator(device=DEV).manual_seed(n * rows)
+    H, T = 8, n * rows
+    unit = lambda: torch.nn.functional.normalize(torch.randn(T, H, 128, generator=g, device=DEV), dim=-1).to(torch.bfloat16)
+    args = [unit(), unit(), unit(), torch.rand(T, H, generator=g, device=DEV) * 0.3 + 0.7, torch.rand(T, H, generator=g, device=DEV)]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    meta, status = [i32(list(range(n))), i32([rows * s for s in range(n)]), i32([rows] * n)], torch.zeros(4, dtype=torch.int32, device=DEV)
+    state0, out = torch.randn(n, H, 128, 128, generator=g, device=DEV) * 0.1, torch.zeros(T, H, 128, dtype=torch.bfloat16, device=DEV)
+    state = state0.clone()
+    call("cuteafd_gated_delta_run", *map(ptr, args), ptr(state), *map(ptr, meta), ptr(out), None, n, H, 0, n, rows, ptr(status), stream())
+    torch.cuda.synchronize()
+    assert status.tolist() == [0, 0, 0, 0]
+    q, k, v, gate, beta = (t.float().cpu() for t in args)
+    for s in (0, n - 1):
+        at = slice(s * rows, (s + 1) * rows)
+        want, final, _ = rops.gated_delta_rule(q[at], k[at], v[at], gate[at], beta[at], state0[s].cpu())
+        assert float((out[at].float().cpu() - want).abs().max()) < 2 ** -8 * float(want.abs().max()) and torch.allclose(state[s].cpu(), final, atol=1e-5, rtol=1e-5)
