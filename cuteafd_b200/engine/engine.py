@@ -368,8 +368,10 @@ class Engine:
 
     def _tiling(self, w, x_act, T: int, f32: bool = False) -> tuple:
         """(operand, split of K) of a dense product.  Steps of 17 to 64 rows, bf16: tiles of 32 rows where a cluster can split K between them in one
-        wave (32 rows x 2048 x 4096: 10 us, against 21 with 64-row tiles and the fix-up through global memory), else 64-row tiles in one piece
-        (12288 x 2048: 15 us, 17 with narrow ones); FP8 always narrow tiles (two CTAs per SM: 1536 x 7168 11 and 29, 24576 x 1536 11 and 42)."""
+        wave (2048 x 4096, 17 and 64 rows: 18 us, against 25 and 37 with 64-row tiles and the fix-up through global memory), else 64-row tiles in one
+        piece (12288 x 2048: 15 us, 17 with narrow ones).  FP8 always narrow tiles: two CTAs per SM, also from 33 rows on, where they read the weights
+        twice (17 / 64 rows, 64-row tiles first: 1536 x 7168 39 / 73 and 19 / 19 us, 24576 x 1536 56 / 66 and 19 / 27, 36864 x 7168 106 / 119 and 57 / 109; the
+        closest is 7168 x 18432 at 33 rows, 86 and 92)."""
         if x_act.tn == 64 and 16 < T <= 64 and w.kind in (KIND_BF16, KIND_FP8B):
             splits = self._splits(w.N, w.K, T, 32, w.kind)
             if splits > 1 or w.kind == KIND_FP8B:
