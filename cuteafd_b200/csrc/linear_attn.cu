@@ -372,7 +372,8 @@ static int short_conv4(const void* x, const float* w, void* carry, const int* sl
   return CA_OK;
 }
 
-// `max_len`: the longest run of the step, which sizes the launch (0: not known, one block walks each sequence).
+// `max_len`: the longest run of the step, which sizes the launch (0: not known, one block walks each sequence).  `update` 0: the carry stays as it is
+// (the verify rows of a speculative step; the accepted ones are replayed with `update` 1, which then moves it).
 extern "C" int cuteafd_short_conv4_run(const void* x, const float* w, void* carry, const int* slot_of_seq, const int* q_start, const int* q_len, void* y, int n_seq, int C, int ldx,
                                        int n_slots, int max_len, int update, int* status, cudaStream_t s) {
   return update ? short_conv4<true>(x, w, carry, slot_of_seq, q_start, q_len, y, n_seq, C, ldx, n_slots, max_len, status, s)
@@ -382,13 +383,6 @@ extern "C" int cuteafd_short_conv4_run(const void* x, const float* w, void* carr
 extern "C" int cuteafd_short_conv4(const void* x, const float* w, void* carry, const int* slot_of_seq, const int* q_start, const int* q_len, void* y,
                                    int n_seq, int C, int ldx, int n_slots, int* status, cudaStream_t s) {
   return short_conv4<true>(x, w, carry, slot_of_seq, q_start, q_len, y, n_seq, C, ldx, n_slots, 0, status, s);
-}
-
-// The same convolution without touching the carry: the verify rows of a speculative step (the accepted prefix is replayed through
-// `cuteafd_short_conv4` afterwards, which then moves the carry).
-extern "C" int cuteafd_short_conv4_peek(const void* x, const float* w, const void* carry, const int* slot_of_seq, const int* q_start, const int* q_len,
-                                        void* y, int n_seq, int C, int ldx, int n_slots, int* status, cudaStream_t s) {
-  return short_conv4<false>(x, w, (void*)carry, slot_of_seq, q_start, q_len, y, n_seq, C, ldx, n_slots, 0, status, s);
 }
 
 // ---------------------------------------------------------------- glue of a gated delta-rule layer

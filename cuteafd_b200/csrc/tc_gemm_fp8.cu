@@ -7,7 +7,7 @@
 // one pipeline stage is exactly one scale block (128 bytes of K per row, four kind::f8f6f4 MMAs of K = 32), each
 // stage accumulates into a FRESH tensor-memory buffer (ring of four), and the epilogue warps pull every finished
 // buffer with tcgen05.ld and add it, scaled, to fp32 registers while the next stages run.  swap-AB as in the other
-// GEMMs (weight rows = MMA M, tokens = MMA N = 16..128), one work unit (128 x TN tile, one K slice) per CTA, optional
+// GEMMs (weight rows = MMA M, tokens = MMA N = 16..64; 128-row token tiles are the wide kernel's), one work unit (128 x TN tile, one K slice) per CTA, optional
 // split-K over a thread-block cluster with the partial tiles reduced through distributed shared memory.
 //
 // Reference counterparts: the W8A8 FP8 GEMV/GEMM (native/shared/cuda/fp8_gemv.cu, fp8_block.cu) and the block-scale
@@ -33,7 +33,7 @@ template <int TN>
 struct Fp8Cfg {
   static constexpr int A_BYTES = 128 * 128, B_BYTES = TN * 128, STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int NACC = 4;
-  static constexpr int TMEM_COLS = NACC * TN < 32 ? 32 : NACC * TN;       // 64 / 128 / 256 / 512
+  static constexpr int TMEM_COLS = NACC * TN < 32 ? 32 : NACC * TN;       // 64 / 128 / 256
   static constexpr int BUDGET = 200 * 1024, MAX_RING = 8;
   static constexpr int SMEM_BYTES = BUDGET + 1024;
   // Shared memory = stage ring + staging area of the cluster reduction + the table of combined scales
@@ -367,8 +367,8 @@ extern "C" int cuteafd_fp8_linear(int tn, const void* tmA, const void* tmB, cons
              "fp8_linear: split-K is up to 4-way for token tiles of up to 64 rows (up to 8-way for 16 rows)");
   if (rows_total <= 0 || N <= 0) return CA_OK;
   const long long items = (rows_total + 127) / 128;
-  // 128-row token tiles: one FMA per output and scale block there, against a shuffle and an FMA here, and double-buffered products (2048 rows x
-  // 7168 x 16384: 302 us, 1361 here; 300 rows x 1536 x 7168, 18 units: 35 us, 75 here)
+  // 128-row token tiles: one FMA per output and scale block in the wide kernel, against a shuffle and an FMA here, and double-buffered products (2048
+  // rows x 7168 x 16384: 302 us, 1361 in the form of this file; 300 rows x 1536 x 7168, 18 units: 35 and 75)
   if (tn == 128) {
     WideArgs wa = {};
     wa.tmX = (const CUtensorMap*)tmB; wa.tmW = (const CUtensorMap*)tmA; wa.sw = sw; wa.sx = sa; wa.Y = Y; wa.R = (const bf16*)R; wa.status = status;
@@ -386,7 +386,6 @@ extern "C" int cuteafd_fp8_linear(int tn, const void* tmA, const void* tmB, cons
     case 16: return fp8_launch<16>(a, grid, stream);
     case 32: return fp8_launch<32>(a, grid, stream);
     case 64: return fp8_launch<64>(a, grid, stream);
-    case 128: return fp8_launch<128>(a, grid, stream);
     default: return ca_fail(CA_ERR_ARG, "fp8_linear: unsupported token tile %d", tn);
   }
 }

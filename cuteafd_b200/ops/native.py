@@ -63,7 +63,6 @@ _PROTOS = {
     "cuteafd_gated_rmsnorm": [P, P, P, P, I, I, I, I, F, P],
     "cuteafd_short_conv4": [P, P, P, P, P, P, P, I, I, I, I, P, P],
     "cuteafd_short_conv4_run": [P, P, P, P, P, P, P, I, I, I, I, I, I, P, P],
-    "cuteafd_short_conv4_peek": [P, P, P, P, P, P, P, I, I, I, I, P, P],
     "cuteafd_mhc_boundary": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, F, P],
     "cuteafd_vision_rgb_patches": [P, P, P, I, I, I, I, I, P],
     "cuteafd_compress_pool": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, F, P],
