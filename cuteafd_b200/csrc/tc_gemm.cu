@@ -1067,14 +1067,20 @@ extern "C" int cuteafd_tc_linear(int kind, int swiglu, int tn, const void* tmA, 
   // 128-row token tiles take the wide kernel from an eighth of the SMs' units (128 tokens x 256 weight rows) on: 4096 bf16 rows x 12288 x 2048 take
   // 160 us there and 420 here, 130 NVFP4 rows x 4096 x 8192 (32 units) 26 and 30, 2331 bf16 rows x 128 x 4096 (19 units) 24 and 26; below, a chain of
   // stages is the same length in both and this kernel's tiles are narrower (1024 rows x 256 x 7168, 8 units: 45 and 41).
-  if (tn == 128 && max_ctas <= 0 && a.splits == 1 && kind != KIND_W4A8 && !peer.n && !grp_rows && act < 2 && !a.trace &&
+  // A split K always goes there and is added up part by part in registers, bit for bit as the fix-up below adds it, without its trip through memory
+  // (flushed L2, parts there / fix-up here / one sum: 130 NVFP4 rows x 4096 x 8192 in 2: 37 / 57 / 37 us, 128 x 9216 x 4096 in 2: 27 / 53 / 25; bf16, 2048 x 128
+  // x 4096 in 8: 37 / 55 / 33, 300 x 2048 x 7168 in 3: 55 / 64 / 55).  Only long bf16 sums of few rows are shorter over many SMs (K 7168 in 8, 65 and
+  // 96 rows x 128: 53 / 37 and 53 / 45, 128 rows: 55 / 53; K 4096, 65 and 96 rows: 37 / 35 and 37 / 43).
+  const bool in_parts = a.splits > 1 && !(kind == KIND_BF16 && rows_total <= 96 && K > 4096);
+  if (tn == 128 && max_ctas <= 0 && (a.splits == 1 || in_parts) && kind != KIND_W4A8 && !peer.n && !grp_rows && act < 2 && !a.trace &&
       (kind == KIND_BF16 || (ldsfb % 16 == 0 && ((uintptr_t)sfb & 15) == 0) || (kind == KIND_MXFP4 && ldsfb % 8 == 0 && ((uintptr_t)sfb & 7) == 0))) {
     const long long items = tiles ? max_tiles : (rows_total + 127) / 128, units = items * (swiglu ? n_nt : (N + 255) / 256);
-    if (8 * units >= ca_sm_count()) {
+    if (in_parts || 8 * units >= ca_sm_count()) {
       WideArgs wa = {};
       wa.tmX = a.tmB; wa.tmW = a.tmA; wa.tmW2 = a.tmA2; wa.sfw = a.sfa; wa.sfw2 = a.sfa2; wa.sfx = a.sfb; wa.ldsfx = ldsfb; wa.alpha = alpha; wa.alpha2 = alpha2;
       wa.tiles = a.tiles; wa.n_tiles = n_tiles; wa.Y = Y; wa.R = a.R; wa.status = status; wa.q_out = a.q_out; wa.sf_out = a.sf_out; wa.inv_gs_out = inv_gs_out;
       wa.ldsf_out = ldsf_out; wa.ldy = ldy; wa.rows_total = rows_total; wa.N = N; wa.K = K; wa.epi = epi; wa.act = act;
+      wa.parts = a.splits;
       return ca_gemm_wide(kind, swiglu != 0, wa, items, stream);
     }
   }

@@ -13,6 +13,7 @@
 // units in flight share a few token tiles and read each expert's weights from HBM once and from L2 after that.
 //   bf16, FP4: a 256-column accumulator.  The epilogue warps first read all of it into registers (128 per thread) and release it, so only
 //   that read (about 400 cycles) lies between two units' MMAs; the arithmetic and the stores run under the next unit's main loop.
+//   Of a K in parts every part is read and added to registers before the next one starts.
 //   FP8: two 256-column buffers; every 128 channels of K is one product of its own, which the epilogue warps add, times its two scales, to
 //   fp32 registers: one FMA per output and scale block, because a thread's row has one activation scale and its 128 columns one weight scale.
 #define CA_PDL_CLASS 1
@@ -74,7 +75,7 @@ __device__ __forceinline__ Unit unit_of(const WideArgs& a, int w, int n_nt) {
 }
 
 // A thread's features n0 .. of one output row, from its accumulators: scale, activation, residual, stores.
-template <int KIND, bool SWIGLU, bool QOUT>
+template <int KIND, bool SWIGLU, bool QOUT, bool PARTS>
 __device__ __forceinline__ void wide_finish(const WideArgs& a, float* acc, int g, size_t row, int n0) {
   constexpr int NF = SWIGLU ? 64 : 128;
   const int nf = min(NF, a.N - n0);
@@ -87,11 +88,11 @@ __device__ __forceinline__ void wide_finish(const WideArgs& a, float* acc, int g
       acc[j] = v / (1.f + __expf(-v)) * up;
     }
   } else {
-    if (KIND != W_FP8) {
+    if (KIND != W_FP8 && !PARTS) {
 #pragma unroll
       for (int j = 0; j < 128; ++j) acc[j] *= al;
     }
-    if (a.act) {
+    if (!PARTS && a.act) {
 #pragma unroll
       for (int j = 0; j < 128; ++j) { const float v = fmaxf(acc[j], 0.f); acc[j] = v * v; }
     }
@@ -174,7 +175,8 @@ __device__ __forceinline__ void wide_finish(const WideArgs& a, float* acc, int g
   }
 }
 
-template <int KIND, bool SWIGLU, bool QOUT>
+// PARTS (an instance of its own: its registers cost the others 2 %): K in a.parts sums.
+template <int KIND, bool SWIGLU, bool QOUT, bool PARTS>
 __global__ void __launch_bounds__(384, 1) gemm_wide_kernel(const __grid_constant__ WideArgs a) {
   using C = WideCfg<KIND>;
   extern __shared__ uint8_t smem_raw[];
@@ -203,6 +205,7 @@ __global__ void __launch_bounds__(384, 1) gemm_wide_kernel(const __grid_constant
   const int n_wb = (a.N + 127) / 128;                                       // 128-row blocks of a weight
   const int nkb = (a.K + C::K_ELEMS - 1) / C::K_ELEMS;
   const int total = n_items * n_nt;
+  const int parts = PARTS ? a.parts : 1;
   volatile int* abortp = &abort_flag;
 
   // Registers: 64,512 at launch (384 x 168); 128 x 64 + 256 x 216 = 63,488 of them after the split.
@@ -239,13 +242,16 @@ __global__ void __launch_bounds__(384, 1) gemm_wide_kernel(const __grid_constant
       if (lane == 0) {
         uint32_t it = 0, tc = 0;
         const uint32_t base = smem_u32(smem);
-        for (int w = blockIdx.x; w < total && !*abortp; w += gridDim.x, ++tc) {
-          bool ok = true;
+        bool ok = true;
+        for (int w = blockIdx.x; ok && w < total && !*abortp; w += gridDim.x)
+        for (int part = 0; part < parts; ++part) {
+          const int kb0 = PARTS ? (int)((long long)nkb * part / parts) : 0, kb1 = PARTS ? (int)((long long)nkb * (part + 1) / parts) : nkb;
+          if (PARTS && kb0 == kb1) continue;
           if (KIND != W_FP8) {
-            if (!mbar_wait_bounded(&acce_bar[0], (tc & 1) ^ 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, w); break; }
+            if (!mbar_wait_bounded(&acce_bar[0], (tc & 1) ^ 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, w); ok = false; break; }
             tc_fence_after();
           }
-          for (int kb = 0; kb < nkb; ++kb, ++it) {
+          for (int kb = kb0; kb < kb1; ++kb, ++it) {
             const int s = it % C::NSTAGE, b = it & 1;
             if (KIND == W_FP8 && !mbar_wait_bounded(&acce_bar[b], ((it >> 1) & 1) ^ 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, w); ok = false; break; }
             if (!mbar_wait_bounded(&full_bar[s], (it / C::NSTAGE) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, w); ok = false; break; }
@@ -263,7 +269,7 @@ __global__ void __launch_bounds__(384, 1) gemm_wide_kernel(const __grid_constant
             const uint64_t xd = umma_desc_sw128(sX), wd = umma_desc_sw128(sW);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-              const uint32_t accum = (KIND == W_FP8 ? k > 0 : (kb > 0 || k > 0)) ? 1u : 0u;
+              const uint32_t accum = (KIND == W_FP8 ? k > 0 : (kb > kb0 || k > 0)) ? 1u : 0u;
               if (KIND == W_BF16) tc_mma_f16(tmem, xd + 2 * k, wd + 2 * k, wide_idesc<KIND>(0), accum);
               else if (KIND == W_FP8) tc_mma_f8(tmem + b * 256, xd + 2 * k, wd + 2 * k, wide_idesc<KIND>(0), accum);
               else if (KIND == W_NVFP4) tc_mma_nvf4(tmem, xd + 2 * k, wd + 2 * k, wide_idesc<KIND>(0), accum, cx + 4 * k, cw + 8 * k);
@@ -273,6 +279,7 @@ __global__ void __launch_bounds__(384, 1) gemm_wide_kernel(const __grid_constant
             if (KIND == W_FP8) tc_commit(&accf_bar[b]);
           }
           if (!ok) break;
+          ++tc;
           if (KIND != W_FP8) tc_commit(&accf_bar[0]);
         }
       }
@@ -329,7 +336,7 @@ __global__ void __launch_bounds__(384, 1) gemm_wide_kernel(const __grid_constant
     const int q4 = warp & 3, h = (warp - 4) >> 2;
     const uint32_t tbase = tmem + ((uint32_t)(q4 * 32) << 16);
     uint32_t it = 0, tc = 0;
-    for (int w = blockIdx.x; w < total; w += gridDim.x, ++tc) {
+    for (int w = blockIdx.x; w < total; w += gridDim.x) {
       if (__any_sync(0xffffffffu, *abortp)) break;                         // the warp stays together
       const Unit u = unit_of(a, w, n_nt);
       const int trow = q4 * 32 + lane;
@@ -388,6 +395,31 @@ __global__ void __launch_bounds__(384, 1) gemm_wide_kernel(const __grid_constant
           for (int e = 0; e < 4; ++e) { sx[e] = sxn[e]; sw[e] = swn[e]; }
         }
         if (!ok) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, w); break; }
+      } else if (PARTS) {
+        // every part times the output scale, one after the other to fp32 registers: the sums that a split over CTAs adds up, without its trip through
+        // memory (the read of a part's accumulator, 400 cycles, is not hidden)
+        const float al = a.alpha ? a.alpha[u.g] : 1.f;
+#pragma unroll
+        for (int j = 0; j < 128; ++j) acc[j] = 0.f;
+        for (int part = 0; part < parts; ++part) {
+          if ((long long)nkb * part / parts == (long long)nkb * (part + 1) / parts) continue;
+          ok = mbar_wait_bounded(&accf_bar[0], tc & 1, abortp);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          tc_fence_after();
+          float p[2][16];
+          tmem_ld_x16(tbase + h * 128, (uint32_t*)p[0]);
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            tc_wait_ld();
+            if (c < 7) tmem_ld_x16(tbase + h * 128 + (c + 1) * 16, (uint32_t*)p[(c + 1) & 1]);
+            else { tc_fence_before(); mbar_arrive(&acce_bar[0]); }
+#pragma unroll
+            for (int j = 0; j < 16; ++j) acc[c * 16 + j] = __fadd_rn(acc[c * 16 + j], __fmul_rn(p[c & 1][j], al));
+          }
+          ++tc;
+        }
+        if (!ok) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_EPILOGUE, w); break; }
       } else {
         ok = mbar_wait_bounded(&accf_bar[0], tc & 1, abortp);
         ok = __all_sync(0xffffffffu, ok);
@@ -399,9 +431,10 @@ __global__ void __launch_bounds__(384, 1) gemm_wide_kernel(const __grid_constant
         tc_wait_ld();
         tc_fence_before();
         mbar_arrive(&acce_bar[0]);
+        ++tc;
       }
       const int n0 = SWIGLU ? u.nt * 128 + h * 64 : u.nt * 256 + h * 128;
-      if (live && n0 < a.N) wide_finish<KIND, SWIGLU, QOUT>(a, acc, u.g, row, n0);
+      if (live && n0 < a.N) wide_finish<KIND, SWIGLU, QOUT, PARTS>(a, acc, u.g, row, n0);
       __syncwarp();
     }
   }
@@ -417,10 +450,10 @@ __global__ void __launch_bounds__(384, 1) gemm_wide_kernel(const __grid_constant
   if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
-template <int KIND, bool SWIGLU, bool QOUT>
+template <int KIND, bool SWIGLU, bool QOUT, bool PARTS = false>
 int launch_wide(const WideArgs& a, int grid, cudaStream_t stream) {
   using C = WideCfg<KIND>;
-  auto kern = gemm_wide_kernel<KIND, SWIGLU, QOUT>;
+  auto kern = gemm_wide_kernel<KIND, SWIGLU, QOUT, PARTS>;
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -437,6 +470,15 @@ int launch_wide(const WideArgs& a, int grid, cudaStream_t stream) {
 int ca_gemm_wide(int kind, bool swiglu, const WideArgs& a, long long max_items, cudaStream_t stream) {
   const long long units = max_items * (swiglu ? (a.N + 127) / 128 : (a.N + 255) / 256);
   const int grid = (int)(units < ca_sm_count() ? (units > 0 ? units : 1) : ca_sm_count());
+  if (a.parts > 1) {
+    if (swiglu || a.tiles || a.act) return ca_fail(CA_ERR_ARG, "gemm_wide: parts of K belong to plain dense products");
+    if (kind == W_BF16) return launch_wide<W_BF16, false, false, true>(a, grid, stream);
+#ifndef CA_TC_BF16_ONLY
+    if (kind == W_NVFP4) return launch_wide<W_NVFP4, false, false, true>(a, grid, stream);
+    if (kind == W_MXFP4) return launch_wide<W_MXFP4, false, false, true>(a, grid, stream);
+#endif
+    return ca_fail(CA_ERR_UNSUPPORTED, "gemm_wide: no kernel in parts for operand kind %d", kind);
+  }
   if (kind == W_BF16) return swiglu ? launch_wide<W_BF16, true, false>(a, grid, stream) : launch_wide<W_BF16, false, false>(a, grid, stream);
 #ifndef CA_TC_BF16_ONLY
   if (kind == W_FP8) return launch_wide<W_FP8, false, false>(a, grid, stream);

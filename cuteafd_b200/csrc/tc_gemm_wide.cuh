@@ -22,6 +22,7 @@ struct WideArgs {
   uint8_t* sf_out;
   const float* inv_gs_out;
   int ldsfx, ldsf_out, ldy, rows_total, N, K, epi, act;
+  int parts;                     // K in this many parts, each a sum of its own, added in order (dense, no activation; 0 and 1: one sum)
 };
 
 // kind: 0 bf16, 1 NVFP4, 2 MXFP4, 3 FP8 with 128-wide fp32 scales.  `max_items`: most token tiles the launch can meet.

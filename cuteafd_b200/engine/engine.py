@@ -356,11 +356,10 @@ class Engine:
                     return s
             return 1
         if tn >= 128 and (kind == KIND_FP8B or (kind == KIND_BF16 and (K <= 2048 or not f32))):
-            # prompt-sized tiles, bf16: the fix-up through global memory costs more than the idle SMs (128-row tiles, 4096 rows x 128 x 2048: 51 us in four parts,
-            # 23 whole; 300 x 2048 x 4096: 59 and 37; 256-row tiles, 300 x 2048 x 4096: 86 and 39).  Long sums that stay fp32 keep their parts: a router
-            # chooses experts by their last bits, and a part rounds less often than one accumulator over all of K (256 x 7168, 4096 rows: 66 us in two
-            # parts, 57 whole).  So do FP4 products (130 rows, 4096 x 8192: 57 and 33), whose results are rounded to four bits next: added in another
-            # order, 150 rows through four layers moved by 0.023, near what their error against 64 bits is.
+            # prompt-sized tiles, bf16: one sum is the shortest (300 x 2048 x 4096: 37 us in 128-row tiles, 39 in 256-row ones, where the fix-up of a split
+            # through global memory takes 86).  Long sums that stay fp32 keep their parts: a router chooses experts by their last bits, and a part rounds
+            # less often than one accumulator over all of K.  So do FP4 products, whose results are rounded to four bits next.  128-row tiles add
+            # their parts up in place (csrc/tc_gemm.cu: 2048 x 256 x 7168 in 4 parts 55 us, 49 as one sum).
             return 1
         # larger token tiles: global-memory fix-up (measured on B200: its cost grows with the split count, the sweet
         # spot is about one work unit per SM and never more than 8 splits)

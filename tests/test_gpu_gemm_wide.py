@@ -102,3 +102,38 @@ def test_wide_expert_products_equal_narrow_ones(kind, counts, N, K):
     ref = torch.nn.functional.silu(xe @ dense[0].T) * (xe @ dense[1].T)
     err = (results[0][1][s:s + max(counts)].double().cpu() - ref).norm() / ref.norm()
     assert float(err) < 2 ** -8                                          # the output's rounding to bf16
+
+
+# (rows, N, K, parts): even and uneven parts, one row and one column block over, K of an unfinished stage, many small parts, an eighth of the SMs and one unit
+PARTS = [(130, 4096, 2048, 2), (65, 512, 4096, 8), (257, 768, 1280, 3), (300, 100, 2336, 4), (129, 288, 1824, 5), (2048, 256, 7168, 4), (1, 256, 1024, 2)]
+
+
+@pytest.mark.parametrize("kind", [KIND_BF16, KIND_NVFP4, KIND_MXFP4])
+@pytest.mark.parametrize("T,N,K,parts", PARTS)
+def test_parts_of_k_are_added_as_a_split_adds_them(kind, T, N, K, parts):
+    """Bit for bit the narrow kernel's fix-up over CTAs (which a limit on the CTAs selects), with every epilogue, and the 64-bit product."""
+    g = torch.Generator(device=DEV).manual_seed(T + N)
+    x = torch.randn(T, K, generator=g, device=DEV).to(torch.bfloat16)
+    w = TcWeight.random(1, N, K, kind, DEV, seed=K)
+    act, st = operand(kind, x, 128), torch.zeros(4, dtype=torch.int32, device=DEV)
+    r = torch.randn(T, N, generator=g, device=DEV).to(torch.bfloat16)
+    for dtype, residual in ((torch.float32, None), (torch.bfloat16, None), (torch.bfloat16, r)):
+        wide, split = (torch.full((T, N), 7.0, dtype=dtype, device=DEV) for _ in range(2))
+        ops.tc_linear(w, act, wide, residual=residual, splits=parts, status=st)
+        ops.tc_linear(w, act, split, residual=residual, splits=parts, max_ctas=148, status=st)
+        torch.cuda.synchronize()
+        assert int(st[0]) == 0
+        assert torch.equal(wide, split)
+        if dtype == torch.float32:
+            ref = dequantised(act) @ w.dequantize()[0].double().T
+            assert float((wide.double().cpu() - ref).norm() / ref.norm()) < 1e-6 * (K / parts) ** 0.5       # fp32 sums of a part's products
+
+
+def test_more_parts_than_stages():
+    """K of three stages in eight parts: five of them are empty."""
+    x = torch.randn(200, 192, device=DEV).to(torch.bfloat16)
+    w, st, y = TcWeight.random(1, 320, 192, KIND_BF16, DEV, seed=3), torch.zeros(4, dtype=torch.int32, device=DEV), torch.zeros(200, 320, device=DEV)
+    ops.tc_linear(w, operand(KIND_BF16, x, 128), y, splits=8, status=st)
+    torch.cuda.synchronize()
+    ref = x.double() @ w.dequantize()[0].double().to(DEV).T
+    assert int(st[0]) == 0 and float((y.double() - ref).norm() / ref.norm()) < 1e-6 * 192 ** 0.5
