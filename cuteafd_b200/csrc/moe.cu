@@ -700,7 +700,8 @@ __global__ void moe_combine_kernel(const bf16* __restrict__ y, const int* __rest
 // the new residual stream `out`, then rmsnorm(out) * norm_w as bf16 (`xn`, optional) and/or quantised to FP4
 // (`q`/`sf`, optional) - three launches (combine, norm, quantise) in one for decode-sized steps.
 // (At most 64 registers: a prompt's launch is bound by its rows' latency, and two blocks of 512 threads per SM hide more of it than one - 4096 tokens
-// x 4096 with 8 routes: 146 us with 72 registers, 82 us.)
+// x 4096 with 8 routes: 146 us with 72 registers, 82 us.  Rows wider than 8192, of 1024 threads with two or four vectors each, cannot launch with more;
+// they spill 96 and 244 bytes.)
 template <int VEC>
 __global__ void __launch_bounds__(1024, 1) moe_combine_norm_kernel(const bf16* __restrict__ y, const int* __restrict__ slot_row, const float* __restrict__ wts,
                                         const bf16* __restrict__ shared, const bf16* __restrict__ residual, bf16* __restrict__ out,

@@ -84,3 +84,20 @@ def test_rows_gathered_quantised_equal_rows_quantised_gathered(kind):
     ops.route_gather(ops.quant_fp4_rows(x, t, inv_gs=gs).data, t.sf, src, n, b, rows, status=st)
     torch.cuda.synchronize()
     assert int(st[0]) == 0 and torch.equal(a.data, b.data) and torch.equal(a.sf, b.sf)
+
+
+@pytest.mark.parametrize("T,H", [(5, 8192), (5, 8200), (3, 9216), (2, 16384), (2, 16392), (2, 32768)])
+def test_combine_with_next_norm_of_wide_rows(T, H):
+    """Rows of one, two and four vectors per thread, at the edges: a block of 1024 threads has 64 registers for each."""
+    k, g = 4, torch.Generator(device=DEV).manual_seed(H)
+    y, w = torch.randn(T * k, H, generator=g, device=DEV).to(torch.bfloat16), torch.rand(H, generator=g, device=DEV) + 0.5
+    slot, wts = torch.randperm(T * k, generator=g, device=DEV).view(T, k).int(), torch.rand(T, k, generator=g, device=DEV)
+    slot[0, 1] = -1
+    x = torch.randn(T, H, generator=g, device=DEV).to(torch.bfloat16)
+    want, got, xn = x.clone(), x.clone(), torch.zeros_like(x)
+    ops.moe_combine(y, slot, wts, None, want, want, T, k)
+    ops.moe_combine(y, slot, wts, None, got, got, T, k, norm_w=w, eps=1e-6, xn=xn)
+    torch.cuda.synchronize()
+    assert torch.equal(want, got)
+    ref = rops.rmsnorm(want.float().cpu(), w.cpu(), 1e-6)
+    assert bool(((xn.float().cpu() - ref).abs() <= 2 ** -8 * ref.abs()).all())              # half a last place of bf16, and fp32 sums
