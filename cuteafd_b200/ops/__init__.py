@@ -78,23 +78,26 @@ def tc_trace(buf: torch.Tensor | None, units: int = 0) -> None:
 
 
 # ------------------------------------------------------------------ TMA descriptors
-def encode_tmap(t: torch.Tensor, box_rows: int, unpack4: bool = False) -> torch.Tensor:
+def encode_tmap(t: torch.Tensor, box_rows: int | tuple, unpack4: bool = False) -> torch.Tensor:
     """Descriptor array (uint8 [G, 128], on t's device) for a K-major operand [G, rows, K] or [rows, K].
     bf16 tensors describe K elements; uint8 tensors describe K bytes (packed fp4 / fp8).  `unpack4`: a uint8 tensor of packed
-    4-bit elements whose tiles TMA expands into 8-bit containers in shared memory (the weight operand of the W4A8 kind)."""
+    4-bit elements whose tiles TMA expands into 8-bit containers in shared memory (the weight operand of the W4A8 kind).
+    Several `box_rows`: [len(box_rows) * G, 128], box by box, in one copy."""
     if t.dim() == 2:
         t = t.unsqueeze(0)
     G, rows, kdim = t.shape
     eb = {torch.bfloat16: 2, torch.uint8: 1}[t.dtype]
     if t.stride(2) != 1:
         raise ValueError("operand must be K-contiguous")
-    host = torch.zeros(G, 128, dtype=torch.uint8)
-    for g in range(G):
+    boxes = box_rows if isinstance(box_rows, tuple) else (box_rows,)
+    host = torch.zeros(len(boxes) * G, 128, dtype=torch.uint8)
+    for i in range(len(boxes) * G):
+        g, box = i % G, boxes[i // G]
         if unpack4:
-            call("cuteafd_tmap_encode_kmajor", host[g].data_ptr(), t[g].data_ptr(), 0, kdim * 2, rows, 1, t.stride(1), 0, box_rows)
+            call("cuteafd_tmap_encode_kmajor", host[i].data_ptr(), t[g].data_ptr(), 0, kdim * 2, rows, 1, t.stride(1), 0, box)
         else:
-            call("cuteafd_tmap_encode_kmajor", host[g].data_ptr(), t[g].data_ptr(), eb, kdim, rows, 1,
-                 t.stride(1) * eb, 0, box_rows)
+            call("cuteafd_tmap_encode_kmajor", host[i].data_ptr(), t[g].data_ptr(), eb, kdim, rows, 1,
+                 t.stride(1) * eb, 0, box)
     return host.to(t.device)
 
 
@@ -244,15 +247,23 @@ class ActBuffer:
     sf: torch.Tensor | None = None
 
     @staticmethod
+    def _tiled(kind: int, tn: int, data: torch.Tensor, sf: torch.Tensor | None = None) -> "ActBuffer":
+        """Over `data`, with the descriptor of `tn` and, for the kinds whose steps of 17 to 64 rows may take 32-row tiles, that one from the same copy."""
+        boxes = (tn, 32) if tn == 64 else (tn,)
+        maps = encode_tmap(data, boxes)
+        act, *rest = (ActBuffer(kind, data.shape[0], data.shape[1], box, data, maps[i:i + 1], sf) for i, box in enumerate(boxes))
+        act.__dict__["_retiled"] = {r.tn: r for r in rest}
+        return act
+
+    @staticmethod
     def alloc(kind: int, rows: int, K: int, tn: int, device) -> "ActBuffer":
         if kind == KIND_BF16:
-            data = torch.zeros(rows, K, dtype=torch.bfloat16, device=device)
-            return ActBuffer(kind, rows, K, tn, data, encode_tmap(data, tn))
+            return ActBuffer._tiled(kind, tn, torch.zeros(rows, K, dtype=torch.bfloat16, device=device))
         if kind == KIND_F32:
             return ActBuffer(kind, rows, K, tn, torch.zeros(rows, K, dtype=torch.float32, device=device), None)
         if kind == KIND_FP8B:    # E4M3 bytes + one fp32 scale per row and 128 channels
             data = torch.zeros(rows, K, dtype=torch.uint8, device=device)
-            return ActBuffer(kind, rows, K, tn, data, encode_tmap(data, tn), torch.zeros(rows, -(-K // 128), dtype=torch.float32, device=device))
+            return ActBuffer._tiled(kind, tn, data, torch.zeros(rows, -(-K // 128), dtype=torch.float32, device=device))
         if kind == KIND_W4A8:    # E4M3 bytes + one UE8M0 scale per row and 32 channels (scale rows padded to whole 128-channel stages)
             data = torch.zeros(rows, K, dtype=torch.uint8, device=device)
             return ActBuffer(kind, rows, K, tn, data, encode_tmap(data, tn), torch.zeros(rows, -(-K // 128) * 4, dtype=torch.uint8, device=device))
@@ -262,7 +273,7 @@ class ActBuffer:
         return ActBuffer(kind, rows, K, tn, data, encode_tmap(data, tn), sf)
 
     def retiled(self, tn: int) -> "ActBuffer":
-        """The same rows in token tiles of `tn` (made once, in the eager run of a new shape)."""
+        """The same rows in token tiles of `tn` (32 of 64: made with the buffer; others once, in the eager run of a new shape)."""
         if tn == self.tn:
             return self
         made = self.__dict__.setdefault("_retiled", {})
@@ -273,7 +284,7 @@ class ActBuffer:
     @staticmethod
     def wrap_bf16(x: torch.Tensor, tn: int) -> "ActBuffer":
         _chk(x, torch.bfloat16, "x")
-        return ActBuffer(KIND_BF16, x.shape[0], x.shape[1], tn, x, encode_tmap(x, tn))
+        return ActBuffer._tiled(KIND_BF16, tn, x)
 
 
 SF_PER_STAGE = {KIND_NVFP4: 16, KIND_MXFP4: 8, KIND_W4A8: 4}        # weight block scales per row and pipeline stage

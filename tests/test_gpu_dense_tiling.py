@@ -36,3 +36,16 @@ def test_dense_products_of_every_tiling(kind, T, N, K):
         xd = (quant.e4m3_decode(act.data.cpu()).reshape(cap, -1, 128) * act.sf.cpu()[:, :, None]).reshape(cap, K).double().to(DEV)
     ref = xd[:T] @ w.dequantize()[0].double().to(DEV).T
     assert float((y[:T].double() - ref).norm() / ref.norm()) < 1e-6 * K ** 0.5       # fp32 sums of K products
+
+
+@pytest.mark.parametrize("kind", [KIND_BF16, KIND_FP8B])
+def test_the_narrow_tiles_of_an_operand_come_with_it(kind):
+    """A new shape's first step allocates and copies nothing for them."""
+    acts = [ActBuffer.alloc(kind, 64, 512, 64, DEV)] + ([ActBuffer.wrap_bf16(torch.zeros(64, 512, dtype=torch.bfloat16, device=DEV), 64)] if kind == KIND_BF16 else [])
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_stats()["allocation.all.allocated"]
+    narrow = [a.retiled(32) for a in acts]
+    assert torch.cuda.memory_stats()["allocation.all.allocated"] == before
+    for a, b in zip(acts, narrow):
+        assert b.tn == 32 and b.data is a.data and b.sf is a.sf and b is a.retiled(32) and a.retiled(64) is a
+        assert torch.equal(b.tmap, ops.encode_tmap(a.data, 32)) and torch.equal(a.tmap, ops.encode_tmap(a.data, 64))
