@@ -6,8 +6,8 @@
 // first expanded once per chunk into per-head keys and values (one GEMM with the kv_b projection, `kvb` below), then
 //   S[128 x 128] = [q_nope | q_rope] [k_nope | k_rope]^T      three 64-wide chunks, tcgen05.mma kind::f16, N = 128 keys
 //   O[128 x 128] += softmax(S) V
-// (a tcgen05.mma of M = 128 costs ~130 cycles whatever its N up to 256, so key tiles are 128 wide: 12 score + 8 PV
-// instructions per 128 keys instead of 24 + 8 with 64-key tiles)
+// (key tiles are 128 wide: 12 score + 8 PV instructions per 128 keys instead of 24 + 8 with 64-key tiles; the tensor pipe is active for 65 cycles
+// of each)
 // with a CTA owning 128 query tokens of ONE head.  k_rope is shared by all heads and comes straight from the gathered latent
 // rows (columns 512..575); k_nope and V come from the expanded buffer [rows, Hl * 256] (per head: 128 key columns, then 128
 // value columns).  Both buffers are contiguous per sequence (`ctx_start[seq]` + key index), so tiles need no page table.
