@@ -18,6 +18,7 @@
 //   fp32 registers: one FMA per output and scale block, because a thread's row has one activation scale and its 128 columns one weight scale.
 #define CA_PDL_CLASS 1
 #include "tc_gemm_wide.cuh"
+#include "tc_issue.cuh"
 
 namespace {
 enum { W_BF16 = 0, W_NVFP4 = 1, W_MXFP4 = 2, W_FP8 = 3 };
@@ -26,6 +27,7 @@ enum { WEPI_BF16 = 0, WEPI_BF16_RESIDUAL = 1, WEPI_F32 = 3 };
 template <int KIND>
 struct WideCfg {
   static constexpr bool FP4 = KIND == W_NVFP4 || KIND == W_MXFP4;
+  static constexpr int ISSUE = KIND == W_BF16 ? TI_F16 : KIND == W_NVFP4 ? TI_NVF4 : KIND == W_MXFP4 ? TI_MXF4 : TI_F8;
   static constexpr int X_BYTES = 128 * 128, W_BYTES = 2 * 128 * 128;
   static constexpr int CHUNKS = KIND == W_NVFP4 ? 4 : (KIND == W_MXFP4 ? 2 : 0);       // 512-byte scale chunks per 128 rows and stage
   static constexpr int SFX_BYTES = CHUNKS * 512, SFW_BYTES = 2 * CHUNKS * 512;
@@ -54,12 +56,12 @@ __device__ __forceinline__ void ld_32b(const void* p, uint32_t* w) {
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) { const bf162 h = __floats2bfloat162_rn(a, b); return *(const uint32_t*)&h; }
 
 template <int KIND>
-__device__ __forceinline__ uint32_t wide_idesc(uint32_t sf_id) {
+__device__ __forceinline__ uint32_t wide_idesc() {
   uint32_t d = ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
   if (KIND == W_BF16) d |= (1u << 4) | (1u << 7) | (1u << 10);             // fp32 accumulator, bf16 x bf16
   else if (KIND == W_FP8) d |= 1u << 4;                                     // fp32 accumulator, E4M3 x E4M3
   else {
-    d |= (sf_id << 4) | (1u << 7) | (1u << 10) | (sf_id << 29);             // E2M1 x E2M1
+    d |= (1u << 7) | (1u << 10);                                            // E2M1 x E2M1
     if (KIND == W_MXFP4) d |= 1u << 23;                                     // UE8M0 scales
   }
   return d;
@@ -184,7 +186,7 @@ __global__ void __launch_bounds__(384, 1) gemm_wide_kernel(const __grid_constant
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::NSTAGE; ++s) { mbar_init(&full_bar[s], C::FP4 ? 33 : 1); mbar_init(&empty_bar[s], 1); }
@@ -239,49 +241,40 @@ __global__ void __launch_bounds__(384, 1) gemm_wide_kernel(const __grid_constant
       __syncwarp();
     } else if (warp == 1) {
       // ---------------------------------------------------------------- MMA issuer
-      if (lane == 0) {
-        uint32_t it = 0, tc = 0;
-        const uint32_t base = smem_u32(smem);
-        bool ok = true;
-        for (int w = blockIdx.x; ok && w < total && !*abortp; w += gridDim.x)
-        for (int part = 0; part < parts; ++part) {
-          const int kb0 = PARTS ? (int)((long long)nkb * part / parts) : 0, kb1 = PARTS ? (int)((long long)nkb * (part + 1) / parts) : nkb;
-          if (PARTS && kb0 == kb1) continue;
-          if (KIND != W_FP8) {
-            if (!mbar_wait_bounded(&acce_bar[0], (tc & 1) ^ 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, w); ok = false; break; }
-            tc_fence_after();
-          }
-          for (int kb = kb0; kb < kb1; ++kb, ++it) {
-            const int s = it % C::NSTAGE, b = it & 1;
-            if (KIND == W_FP8 && !mbar_wait_bounded(&acce_bar[b], ((it >> 1) & 1) ^ 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, w); ok = false; break; }
-            if (!mbar_wait_bounded(&full_bar[s], (it / C::NSTAGE) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, w); ok = false; break; }
-            tc_fence_after();
-            const uint32_t sX = base + s * C::STAGE_BYTES, sW = sX + C::X_BYTES, sSX = sW + C::W_BYTES, sSW = sSX + C::SFX_BYTES;
-            const uint32_t cx = tmem + C::SF_COL + b * 64, cw = cx + 16;
-            if (C::FP4) {
-#pragma unroll
-              for (int q = 0; q < C::CHUNKS; ++q) {
-                tc_cp_sf(cx + 4 * q, umma_desc_sf(sSX + q * 512));
-                tc_cp_sf(cw + 8 * q, umma_desc_sf(sSW + q * 512));
-                tc_cp_sf(cw + 8 * q + 4, umma_desc_sf(sSW + C::SFX_BYTES + q * 512));
-              }
-            }
-            const uint64_t xd = umma_desc_sw128(sX), wd = umma_desc_sw128(sW);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const uint32_t accum = (KIND == W_FP8 ? k > 0 : (kb > kb0 || k > 0)) ? 1u : 0u;
-              if (KIND == W_BF16) tc_mma_f16(tmem, xd + 2 * k, wd + 2 * k, wide_idesc<KIND>(0), accum);
-              else if (KIND == W_FP8) tc_mma_f8(tmem + b * 256, xd + 2 * k, wd + 2 * k, wide_idesc<KIND>(0), accum);
-              else if (KIND == W_NVFP4) tc_mma_nvf4(tmem, xd + 2 * k, wd + 2 * k, wide_idesc<KIND>(0), accum, cx + 4 * k, cw + 8 * k);
-              else tc_mma_mxf4(tmem, xd + 2 * k, wd + 2 * k, wide_idesc<KIND>((k & 1) * 2), accum, cx + 4 * (k >> 1), cw + 8 * (k >> 1));
-            }
-            tc_commit(&empty_bar[s]);
-            if (KIND == W_FP8) tc_commit(&accf_bar[b]);
-          }
-          if (!ok) break;
-          ++tc;
-          if (KIND != W_FP8) tc_commit(&accf_bar[0]);
+      // (the whole warp, under an elected lane's predicate: tc_issue.cuh)
+      uint32_t it = 0, tc = 0;
+      const uint32_t x0 = ti_desc(smem_u32(smem)), sx0 = ti_desc_sf(smem_u32(smem) + C::X_BYTES + C::W_BYTES);
+      bool ok = true;
+      for (int w = blockIdx.x; ok && w < total && !__any_sync(0xffffffffu, *abortp); w += gridDim.x)
+      for (int part = 0; part < parts; ++part) {
+        const int kb0 = PARTS ? (int)((long long)nkb * part / parts) : 0, kb1 = PARTS ? (int)((long long)nkb * (part + 1) / parts) : nkb;
+        if (PARTS && kb0 == kb1) continue;
+        if (KIND != W_FP8) {
+          if (!mbar_wait_warp(&acce_bar[0], (tc & 1) ^ 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, w); ok = false; break; }
+          tc_fence_after();
         }
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+          const uint32_t s = it % C::NSTAGE, b = it & 1;
+          if (KIND == W_FP8 && !mbar_wait_warp(&acce_bar[b], ((it >> 1) & 1) ^ 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, w); ok = false; break; }
+          if (!mbar_wait_warp(&full_bar[s], (it / C::NSTAGE) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, w); ok = false; break; }
+          tc_fence_after();
+          const uint32_t off = s * (C::STAGE_BYTES / 16), cx = tmem + C::SF_COL + b * 64, cw = cx + 16;
+          if (C::FP4) {
+#pragma unroll
+            for (int q = 0; q < C::CHUNKS; ++q) {
+              const uint32_t chunk = sx0 + off + q * 32;
+              ti_cp_sf(cx + 4 * q, chunk);
+              ti_cp_sf(cw + 8 * q, chunk + C::SFX_BYTES / 16);
+              ti_cp_sf(cw + 8 * q + 4, chunk + C::SFX_BYTES / 8);
+            }
+          }
+          ti_mma4<C::ISSUE, 4, 8>(tmem + (KIND == W_FP8 ? b * 256 : 0), x0 + off, x0 + off + C::X_BYTES / 16, wide_idesc<KIND>(), KIND == W_FP8 ? 0u : (kb > kb0 ? 1u : 0u), cx, cw);
+          ti_commit(&empty_bar[s]);
+          if (KIND == W_FP8) ti_commit(&accf_bar[b]);
+        }
+        if (!ok) break;
+        ++tc;
+        if (KIND != W_FP8) ti_commit(&accf_bar[0]);
       }
       __syncwarp();
     } else if (warp == 2 && C::FP4) {
