@@ -25,6 +25,7 @@
 
 #define CA_PDL_CLASS 2
 #include "common.cuh"
+#include "tc_issue.cuh"
 
 #define MKEYS 64            // keys per tile = one page
 #define MPAGE 64
@@ -104,7 +105,7 @@ __global__ void __launch_bounds__(192, MlaGeo<NC, NL>::OCC) mla_attn_kernel(cons
   uint32_t& tmem_slot = *(uint32_t*)(bars + 2 * NST_ + 4);
   int& abort_flag = *(int*)(bars + 2 * NST_ + 5);
   if (smem_u32(smem) & 1023) { if (threadIdx.x == 0) ca_dev_fail(a.status, CA_DEV_BAD_INDEX, 0xA12); return; }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, tid = threadIdx.x;
 
   const int tok_per_tile = 128 / a.Hl;
   const int split = blockIdx.x, vh = blockIdx.y;
@@ -194,59 +195,47 @@ __global__ void __launch_bounds__(192, MlaGeo<NC, NL>::OCC) mla_attn_kernel(cons
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     const uint32_t id_s = mla_idesc(MKEYS, 0), id_o = mla_idesc(nv * 64, 1);
-    // One thread issues everything.  It polls two conditions and serves whichever is ready: "the latent tile qk has
-    // landed and the score buffer is free" (issue its scores) and "the probabilities of tile pv are in shared memory"
-    // (issue its PV product, which also releases the tile's stage to the producer).  The 36 score MMAs of a tile
-    // keep the issuing thread busy for as long as they execute (~130 cycles each whatever their operands, so a tile
-    // is 64 keys wide to halve the count per key), and the PV probe is repeated between the 64-wide chunks:
-    // otherwise a PV product that became ready just after the scores started would wait a whole score pass, and with
-    // it the stage release and the next load.
+    // One warp issues everything, under an elected lane's predicate (tc_issue.cuh).  It polls two conditions and serves whichever is ready: "the
+    // latent tile qk has landed and the score buffer is free" (issue its scores) and "the probabilities of tile pv are in shared memory"
+    // (issue its PV product, which also releases the tile's stage to the producer).  The 36 score products of a tile fill the tensor pipe's queue, so
+    // issuing them takes as long as they do; the PV probe is repeated between the 64-wide chunks: otherwise a PV product that became ready just after
+    // the scores started would wait a whole score pass, and with it the stage release and the next load.
     // There is one score buffer: the softmax threads copy it to registers first thing and release it (s_free).
-    if (lane == 0) {
-      int qk = 0, pv = 0, idle = 0;
-      long long idle_t0 = 0;
-      auto try_pv = [&]() -> bool {
-        if (pv >= qk || !mbar_test(&p_full, pv & 1)) return false;
+    const uint32_t kd = ti_desc(smem_u32(sK)), qd = ti_desc(smem_u32(sQ)), pd = (uint32_t)mla_desc_k_plain(smem_u32(sP), 128, MKEYS * 16);
+    const uint32_t vd = (uint32_t)mla_desc_mn_sw128(smem_u32(sK) + (G::VCH * vh) * SK_CHUNK, SK_CHUNK, 1024);
+    auto ready = [](uint64_t* bar, int ph) { return __all_sync(0xffffffffu, mbar_test(bar, ph & 1)); };
+    int qk = 0, pv = 0, idle = 0;
+    long long idle_t0 = 0;
+    auto try_pv = [&]() -> bool {
+      if (pv >= qk || !ready(&p_full, pv)) return false;
+      tc_fence_after();
+      const int s = pv % NST_;
+      ti_f16x4_ss<16, 128, 0x4000 | MKEYS>(tmem + O_COL, pd, vd + s * (G::STAGE / 16), id_o, pv);       // 16 keys per product: two 8-key groups = 2048 B along K
+      ti_commit(&k_empty[s]);
+      ti_commit(&o_done);
+      ++pv;
+      return true;
+    };
+    while (pv < n_tiles) {
+      bool did = try_pv();
+      if (qk < n_tiles && (qk == 0 || ready(&s_free, qk - 1)) && ready(&k_full[qk % NST_], qk / NST_)) {
         tc_fence_after();
-        const int s = pv % NST_;
-        const uint32_t v0 = smem_u32(sK + s * G::STAGE) + (G::VCH * vh) * SK_CHUNK;
-#pragma unroll
-        for (int k = 0; k < MKEYS / 16; ++k)       // 16 keys per MMA: two 8-key groups = 2048 B along K
-          tc_mma_f16(tmem + O_COL, mla_desc_k_plain(smem_u32(sP) + k * 256, 128, MKEYS * 16), mla_desc_mn_sw128(v0 + k * 2048, SK_CHUNK, 1024), id_o,
-                     (pv | k) ? 1u : 0u);
-        tc_commit(&k_empty[s]);
-        tc_commit(&o_done);
-        ++pv;
-        return true;
-      };
-      while (pv < n_tiles) {
-        bool did = try_pv();
-        if (qk < n_tiles && (qk == 0 || mbar_test(&s_free, (qk - 1) & 1)) && mbar_test(&k_full[qk % NST_], (qk / NST_) & 1)) {
-          tc_fence_after();
-          const uint32_t k0 = smem_u32(sK + (qk % NST_) * G::STAGE), d = tmem + S_COL;
+        const uint32_t k0 = kd + (qk % NST_) * (G::STAGE / 16), d = tmem + S_COL;
 #pragma unroll 1
-          for (int c = 0; c < NC; ++c) {
-            if (c < G::QT) {
-#pragma unroll
-              for (int k = 0; k < 4; ++k)
-                tc_mma_f16_ta(d, tmem + QT_COL + c * 32 + k * 8, mla_desc_k_sw128(k0 + c * SK_CHUNK) + 2 * k, id_s, (c | k) ? 1u : 0u);
-            } else {
-#pragma unroll
-              for (int k = 0; k < 4; ++k)
-                tc_mma_f16(d, mla_desc_k_sw128(smem_u32(sQ) + (c - G::QT) * 16384) + 2 * k, mla_desc_k_sw128(k0 + c * SK_CHUNK) + 2 * k, id_s, 1u);
-            }
-            if (c + 1 < NC) try_pv();
-          }
-          tc_commit(&s_full);
-          ++qk;
-          did = true;
+        for (int c = 0; c < NC; ++c) {
+          if (c < G::QT) ti_f16x4_ts<2>(d, tmem + QT_COL + c * 32, k0 + c * (SK_CHUNK / 16), id_s, c);
+          else ti_mma4<TI_F16>(d, qd + (c - G::QT) * 1024, k0 + c * (SK_CHUNK / 16), id_s, 1u);
+          if (c + 1 < NC) try_pv();
         }
-        if (did) { idle = 0; continue; }
-        if (idle++ == 0) idle_t0 = clock64();
-        if ((idle & 255) == 0) {
-          if (*abortp) break;
-          if (clock64() - idle_t0 > 4000000000LL) { *abortp = 1; ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, pv); break; }
-        }
+        ti_commit(&s_full);
+        ++qk;
+        did = true;
+      }
+      if (did) { idle = 0; continue; }
+      if (idle++ == 0) idle_t0 = clock64();
+      if ((idle & 255) == 0) {
+        if (__any_sync(0xffffffffu, *abortp)) break;
+        if (__any_sync(0xffffffffu, clock64() - idle_t0 > 4000000000LL)) { *abortp = 1; ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, pv); break; }
       }
     }
     __syncwarp();
@@ -424,7 +413,7 @@ __global__ void __launch_bounds__(192, 1) mla_attn_pair_kernel(const __grid_cons
   uint64_t* x_full = bars + 2 * PNST + 4;                 // [2]: the partner's partial scores of tile i landed in sX[i & 1]
   uint32_t& tmem_slot = *(uint32_t*)(bars + 2 * PNST + 6);
   int& abort_flag = *(int*)(bars + 2 * PNST + 7);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, tid = threadIdx.x;
   const bool aligned = (smem_u32(smem) & 1023) == 0;       // same answer in both CTAs of the pair (same kernel, same layout)
 
   const int tok_per_tile = 128 / a.Hl;
@@ -510,47 +499,42 @@ __global__ void __launch_bounds__(192, 1) mla_attn_pair_kernel(const __grid_cons
       __syncwarp();
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer (one thread; see mla_attn_kernel)
+    // ------------------------------------------------------------------ MMA issuer (see mla_attn_kernel)
     const uint32_t id_s = mla_idesc(MKEYS, 0), id_o = mla_idesc(256, 1);
-    if (lane == 0) {
-      int qk = 0, pv = 0, idle = 0;
-      long long idle_t0 = 0;
-      auto try_pv = [&]() -> bool {
-        if (pv >= qk || !mbar_test(&p_full, pv & 1)) return false;
+    const uint32_t kd = ti_desc(smem_u32(sK)), pd = (uint32_t)mla_desc_k_plain(smem_u32(sP), 128, MKEYS * 16);
+    const uint32_t vd = (uint32_t)mla_desc_mn_sw128(smem_u32(sK), SK_CHUNK, 1024);           // the V half is the first four chunks of the stage in both CTAs
+    auto ready = [](uint64_t* bar, int ph) { return __all_sync(0xffffffffu, mbar_test(bar, ph & 1)); };
+    int qk = 0, pv = 0, idle = 0;
+    long long idle_t0 = 0;
+    auto try_pv = [&]() -> bool {
+      if (pv >= qk || !ready(&p_full, pv)) return false;
+      tc_fence_after();
+      const int s = pv % PNST;
+      ti_f16x4_ss<16, 128, 0x4000 | MKEYS>(tmem + O_COL, pd, vd + s * (PK_STAGE / 16), id_o, pv);       // 16 keys per product: two 8-key groups = 2048 B along K
+      ti_commit(&k_empty[s]);
+      ti_commit(&o_done);
+      ++pv;
+      return true;
+    };
+    while (pv < n_tiles) {
+      bool did = try_pv();
+      if (qk < n_tiles && (qk == 0 || ready(&s_free, qk - 1)) && ready(&k_full[qk % PNST], qk / PNST)) {
         tc_fence_after();
-        const int s = pv % PNST;
-        const uint32_t v0 = smem_u32(sK + s * PK_STAGE);           // the V half is the first four chunks of the stage in both CTAs
-#pragma unroll
-        for (int k = 0; k < MKEYS / 16; ++k)
-          tc_mma_f16(tmem + O_COL, mla_desc_k_plain(smem_u32(sP) + k * 256, 128, MKEYS * 16), mla_desc_mn_sw128(v0 + k * 2048, SK_CHUNK, 1024), id_o,
-                     (pv | k) ? 1u : 0u);
-        tc_commit(&k_empty[s]);
-        tc_commit(&o_done);
-        ++pv;
-        return true;
-      };
-      while (pv < n_tiles) {
-        bool did = try_pv();
-        if (qk < n_tiles && (qk == 0 || mbar_test(&s_free, (qk - 1) & 1)) && mbar_test(&k_full[qk % PNST], (qk / PNST) & 1)) {
-          tc_fence_after();
-          const uint32_t k0 = smem_u32(sK + (qk % PNST) * PK_STAGE), d = tmem + S_COL;
+        const uint32_t k0 = kd + (qk % PNST) * (PK_STAGE / 16), d = tmem + S_COL;
 #pragma unroll 1
-          for (int c = c_lo; c < c_hi; ++c) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              tc_mma_f16_ta(d, tmem + QT_COL + (c - c_lo) * 32 + k * 8, mla_desc_k_sw128(k0 + (c - l_lo) * SK_CHUNK) + 2 * k, id_s, ((c - c_lo) | k) ? 1u : 0u);
-            if (c + 1 < c_hi) try_pv();
-          }
-          tc_commit(&s_full);
-          ++qk;
-          did = true;
+        for (int c = c_lo; c < c_hi; ++c) {
+          ti_f16x4_ts<2>(d, tmem + QT_COL + (c - c_lo) * 32, k0 + (c - l_lo) * (SK_CHUNK / 16), id_s, c - c_lo);
+          if (c + 1 < c_hi) try_pv();
         }
-        if (did) { idle = 0; continue; }
-        if (idle++ == 0) idle_t0 = clock64();
-        if ((idle & 255) == 0) {
-          if (*abortp) break;
-          if (clock64() - idle_t0 > 4000000000LL) { *abortp = 1; ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, pv); break; }
-        }
+        ti_commit(&s_full);
+        ++qk;
+        did = true;
+      }
+      if (did) { idle = 0; continue; }
+      if (idle++ == 0) idle_t0 = clock64();
+      if ((idle & 255) == 0) {
+        if (__any_sync(0xffffffffu, *abortp)) break;
+        if (__any_sync(0xffffffffu, clock64() - idle_t0 > 4000000000LL)) { *abortp = 1; ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, pv); break; }
       }
     }
     __syncwarp();

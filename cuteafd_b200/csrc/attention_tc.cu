@@ -27,6 +27,7 @@
 
 #define CA_PDL_CLASS 2
 #include "common.cuh"
+#include "tc_issue.cuh"
 #include "attn_common.cuh"
 #include "attn_extras.cuh"
 
@@ -140,7 +141,7 @@ __global__ void __launch_bounds__(192, AttnTcCfg<KC, VC>::OCC) paged_attn_tc_ker
   uint8_t* sP = smem + Cf::Q_BYTES;         // [128 rows x 128 B]
   uint8_t* sK = smem + Cf::K_OFF;           // 2 stages x KC x 8 KB
   uint8_t* sV = smem + Cf::V_OFF;           // 2 stages x VC x 8 KB
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, tid = threadIdx.x;
 
   const int G = a.Hq / a.Hkv;
   const int tok_per_tile = 128 / G;
@@ -247,40 +248,29 @@ __global__ void __launch_bounds__(192, AttnTcCfg<KC, VC>::OCC) paged_attn_tc_ker
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     // Scores are double-buffered in tensor memory: S(i+1) is computed while the softmax of tile i runs.
+    // The whole warp waits and issues under an elected lane's predicate (tc_issue.cuh).
     const uint32_t id_s = idesc_bf16(64, 0), id_o = idesc_bf16(VC * 64, 1);
+    const uint32_t qd = ti_desc(smem_u32(sQ)), kd = ti_desc(smem_u32(sK)), pd = ti_desc(smem_u32(sP)), vd = (uint32_t)desc_mnmajor_sw128(smem_u32(sV), 8192, 1024);
     auto issue_scores = [&](int j) -> bool {     // S[j & 1] = Q K(j)^T
       const int s = j & 1;
-      if (!mbar_wait_bounded(&k_full[s], (j >> 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, j); return false; }
+      if (!mbar_wait_warp(&k_full[s], (j >> 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, j); return false; }
       tc_fence_after();
-      if (lane == 0) {
-        const uint32_t k0 = smem_u32(sK + s * Cf::K_STAGE), d = tmem + (s ? S1_COL : S0_COL);
 #pragma unroll
-        for (int kb = 0; kb < KC; ++kb)
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            tc_mma_f16(d, desc_kmajor_sw128(smem_u32(sQ) + kb * 16384) + 2 * k, desc_kmajor_sw128(k0 + kb * 8192) + 2 * k, id_s, (kb | k) ? 1u : 0u);
-        tc_commit(&s_full[s]);
-        tc_commit(&k_empty[s]);
-      }
-      __syncwarp();
+      for (int kb = 0; kb < KC; ++kb) ti_mma4<TI_F16>(tmem + (s ? S1_COL : S0_COL), qd + kb * 1024, kd + s * (Cf::K_STAGE / 16) + kb * 512, id_s, kb);
+      ti_commit(&s_full[s]);
+      ti_commit(&k_empty[s]);
       return true;
     };
     bool ok = true;
     for (int j = 0; ok && j < min(2, n_tiles); ++j) ok = issue_scores(j);
     for (int i = 0; ok && i < n_tiles; ++i) {
       const int s = i & 1;
-      if (!mbar_wait_bounded(&p_full, i & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, i); break; }
-      if (!mbar_wait_bounded(&v_full[s], (i >> 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, i); break; }
+      if (!mbar_wait_warp(&p_full, i & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, i); break; }
+      if (!mbar_wait_warp(&v_full[s], (i >> 1) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, i); break; }
       tc_fence_after();
-      if (lane == 0) {
-        const uint32_t v0 = smem_u32(sV + s * Cf::V_STAGE);
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          tc_mma_f16(tmem + O_COL, desc_kmajor_sw128(smem_u32(sP)) + 2 * k, desc_mnmajor_sw128(v0 + k * 2048, 8192, 1024), id_o, (i | k) ? 1u : 0u);
-        tc_commit(&v_empty[s]);
-        tc_commit(&o_done);
-      }
-      __syncwarp();
+      ti_f16x4_ss<2, 128>(tmem + O_COL, pd, vd + s * (Cf::V_STAGE / 16), id_o, i);       // 16 keys of V are 2,048 bytes
+      ti_commit(&v_empty[s]);
+      ti_commit(&o_done);
       if (i + 2 < n_tiles) ok = issue_scores(i + 2);   // S[i & 1] was consumed before p_full(i) completed
     }
   } else if ((warp & 3) >= n_live_warps) {

@@ -24,6 +24,7 @@
 #define CA_PDL_CLASS 1
 #include <stdlib.h>
 #include "tc_gemm_wide.cuh"
+#include "tc_issue.cuh"
 
 // KIND_W4A8: MXFP4 weights (E2M1 + UE8M0 / 32, unpacked by TMA into 8-bit containers) x FP8 E4M3 activations with UE8M0 / 32
 // scales, kind::mxf8f6f4 (K = 32 per instruction) - the reference's default expert arithmetic
@@ -86,6 +87,7 @@ struct TcArgs {
 template <int KIND, int TN, bool SWIGLU>
 struct TcCfg {
   static constexpr int NA = SWIGLU ? 2 : 1;
+  static constexpr int ISSUE = KIND == KIND_BF16 ? TI_F16 : KIND == KIND_NVFP4 ? TI_NVF4 : KIND == KIND_MXFP4 ? TI_MXF4 : TI_W4A8;
   static constexpr int A_BYTES = 128 * 128;
   static constexpr int B_BYTES = TN * 128;
   static constexpr int NBLK = TN > 128 ? 2 : 1;                      // 128-token scale blocks
@@ -183,7 +185,7 @@ __global__ void __launch_bounds__(192, TcCfg<KIND, TN, SWIGLU>::OCC) tc_linear_k
   __shared__ int abort_flag;
 
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::NSTAGE; ++s) { mbar_init(&full_bar[s], 33); mbar_init(&empty_bar[s], 1); }   // 1 expect_tx + 32 lanes
@@ -285,66 +287,42 @@ __global__ void __launch_bounds__(192, TcCfg<KIND, TN, SWIGLU>::OCC) tc_linear_k
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    // One elected thread waits and issues (the other lanes park at the warp barrier below): no per-stage
-    // divergence or reconvergence on the chain that bounds a decode-sized tile.
-    if (lane == 0) {
-      uint32_t it = 0, tc = 0;
-      const uint32_t smem_base = smem_u32(smem);
-      for (int w = w_begin; w < w_end && !*abortp; ++w, ++tc) {
-        const int sp = w % splits;
-        const int kb0 = (int)(((long long)nkb_all * sp) / splits), kb1 = (int)(((long long)nkb_all * (sp + 1)) / splits);
-        const int acc = tc % C::NACC;
-        if (!mbar_wait_bounded(&acce_bar[acc], ((tc / C::NACC) & 1) ^ 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, w); break; }
+    // The whole warp waits and issues under an elected lane's predicate (tc_issue.cuh).
+    uint32_t it = 0, tc = 0;
+    const uint32_t desc0 = ti_desc(smem_u32(smem)), sf0 = ti_desc_sf(smem_u32(smem) + C::NA * C::A_BYTES + C::B_BYTES);
+    for (int w = w_begin; w < w_end && !__any_sync(0xffffffffu, *abortp); ++w, ++tc) {
+      const int sp = w % splits;
+      const int kb0 = (int)(((long long)nkb_all * sp) / splits), kb1 = (int)(((long long)nkb_all * (sp + 1)) / splits);
+      const int acc = tc % C::NACC;
+      if (!mbar_wait_warp(&acce_bar[acc], ((tc / C::NACC) & 1) ^ 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, w); break; }
+      tc_fence_after();
+      TC_TRACE(2, clock64());
+      const uint32_t d0 = tmem + acc * C::ACC_COLS;
+      bool ok = true;
+      for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        const uint32_t s = it % C::NSTAGE;
+        if (!mbar_wait_warp(&full_bar[s], (it / C::NSTAGE) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, w); ok = false; break; }
         tc_fence_after();
-        TC_TRACE(2, clock64());
-        const uint32_t d0 = tmem + acc * C::ACC_COLS;
-        bool ok = true;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = it % C::NSTAGE;
-          if (!mbar_wait_bounded(&full_bar[s], (it / C::NSTAGE) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, w); ok = false; break; }
-          tc_fence_after();
-          if (KIND != KIND_BF16) fence_proxy_async_smem();   // scale bytes arrived through the generic proxy (cp.async)
-          const uint32_t st = smem_base + s * C::STAGE_BYTES;
-          const uint32_t sA = st, sB = st + C::NA * C::A_BYTES, sSFA = sB + C::B_BYTES, sSFB = sSFA + C::NA * C::SFA_BYTES;
-          if (KIND != KIND_BF16) {
+        if (KIND != KIND_BF16) fence_proxy_async_smem();   // scale bytes arrived through the generic proxy (cp.async)
+        const uint32_t off = s * (C::STAGE_BYTES / 16), dA = desc0 + off, dB = dA + C::NA * C::A_BYTES / 16;
+        if (KIND != KIND_BF16) {
+          const uint32_t sfa = sf0 + off, sfb = sfa + C::NA * C::SFA_BYTES / 16;
 #pragma unroll
-            for (int q = 0; q < C::SF_CHUNKS; ++q) {
-              tc_cp_sf(tmem + C::SFA_COL + 4 * q, umma_desc_sf(sSFA + q * 512));
-              if (SWIGLU) tc_cp_sf(tmem + C::SFA2_COL + 4 * q, umma_desc_sf(sSFA + C::SFA_BYTES + q * 512));
+          for (int q = 0; q < C::SF_CHUNKS; ++q) {
+            ti_cp_sf(tmem + C::SFA_COL + 4 * q, sfa + q * 32);
+            if (SWIGLU) ti_cp_sf(tmem + C::SFA2_COL + 4 * q, sfa + C::SFA_BYTES / 16 + q * 32);
 #pragma unroll
-              for (int b = 0; b < C::NBLK; ++b)
-                tc_cp_sf(tmem + C::SFB_COL + (4 * C::NBLK) * q + 4 * b, umma_desc_sf(sSFB + b * (C::SF_CHUNKS * 512) + q * 512));
-            }
+            for (int b = 0; b < C::NBLK; ++b) ti_cp_sf(tmem + C::SFB_COL + (4 * C::NBLK) * q + 4 * b, sfb + (b * C::SF_CHUNKS + q) * 32);
           }
-          const uint64_t adesc = umma_desc_sw128(sA), a2desc = umma_desc_sw128(sA + C::A_BYTES), bdesc = umma_desc_sw128(sB);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const uint32_t accum = (kb > kb0 || k > 0) ? 1u : 0u;
-            if (KIND == KIND_BF16) {
-              const uint32_t id = make_idesc(KIND_BF16, TN, 0);
-              tc_mma_f16(d0, adesc + 2 * k, bdesc + 2 * k, id, accum);
-              if (SWIGLU) tc_mma_f16(d0 + TN, a2desc + 2 * k, bdesc + 2 * k, id, accum);
-            } else if (KIND == KIND_NVFP4) {
-              const uint32_t id = make_idesc(KIND_NVFP4, TN, 0);
-              tc_mma_nvf4(d0, adesc + 2 * k, bdesc + 2 * k, id, accum, tmem + C::SFA_COL + 4 * k, tmem + C::SFB_COL + 4 * C::NBLK * k);
-              if (SWIGLU) tc_mma_nvf4(d0 + TN, a2desc + 2 * k, bdesc + 2 * k, id, accum, tmem + C::SFA2_COL + 4 * k, tmem + C::SFB_COL + 4 * C::NBLK * k);
-            } else if (KIND == KIND_W4A8) {
-              const uint32_t id = make_idesc(KIND_W4A8, TN, k);       // one scale column per stage, byte k of it per K = 32 step
-              tc_mma_mxf8f6f4(d0, adesc + 2 * k, bdesc + 2 * k, id, accum, tmem + C::SFA_COL, tmem + C::SFB_COL);
-              if (SWIGLU) tc_mma_mxf8f6f4(d0 + TN, a2desc + 2 * k, bdesc + 2 * k, id, accum, tmem + C::SFA2_COL, tmem + C::SFB_COL);
-            } else {
-              const uint32_t id = make_idesc(KIND_MXFP4, TN, (k & 1) * 2);
-              const int q = k >> 1;
-              tc_mma_mxf4(d0, adesc + 2 * k, bdesc + 2 * k, id, accum, tmem + C::SFA_COL + 4 * q, tmem + C::SFB_COL + 4 * C::NBLK * q);
-              if (SWIGLU) tc_mma_mxf4(d0 + TN, a2desc + 2 * k, bdesc + 2 * k, id, accum, tmem + C::SFA2_COL + 4 * q, tmem + C::SFB_COL + 4 * C::NBLK * q);
-            }
-          }
-          tc_commit(&empty_bar[s]);
         }
-        if (!ok) break;
-        tc_commit(&accf_bar[acc]);
-        TC_TRACE(4, clock64());
+        const uint32_t id = make_idesc(KIND, TN, 0), accum = kb > kb0 ? 1u : 0u;
+        ti_mma4<C::ISSUE, 4, 4 * C::NBLK>(d0, dA, dB, id, accum, tmem + C::SFA_COL, tmem + C::SFB_COL);
+        if (SWIGLU) ti_mma4<C::ISSUE, 4, 4 * C::NBLK>(d0 + TN, dA + C::A_BYTES / 16, dB, id, accum, tmem + C::SFA2_COL, tmem + C::SFB_COL);
+        ti_commit(&empty_bar[s]);
       }
+      if (!ok) break;
+      ti_commit(&accf_bar[acc]);
+      TC_TRACE(4, clock64());
     }
     __syncwarp();
   } else {
@@ -677,7 +655,7 @@ __global__ void __launch_bounds__(192, 1) tc_linear_cluster_kernel(const __grid_
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int S = a.splits;
   float* staging = (float*)(smem + L::ring(S) * C::STAGE_BYTES);         // [S-1][TN][128] fp32, rank 0's copy is the one used
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     CL_TRACE(0);
@@ -748,42 +726,29 @@ __global__ void __launch_bounds__(192, 1) tc_linear_cluster_kernel(const __grid_
       }
     }
   } else if (warp == 1) {
-    // ---- MMA issuer (one elected thread)
+    // ---- MMA issuer (the warp, under an elected lane's predicate: tc_issue.cuh)
     pdl_wait();
-    if (lane == 0) {
-      const uint32_t smem_base = smem_u32(smem);
-      bool ok = true;
-      for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
-        const int s = it % ring;
-        if (!mbar_wait_bounded(&full_bar[s], (it / ring) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, (int)blockIdx.x); ok = false; break; }
-        if (it == 0) CL_TRACE(3);
-        tc_fence_after();
-        if (KIND != KIND_BF16) fence_proxy_async_smem();
-        const uint32_t st = smem_base + s * C::STAGE_BYTES;
-        const uint32_t sA = st, sB = st + C::A_BYTES, sSFA = sB + C::B_BYTES, sSFB = sSFA + C::SFA_BYTES;
-        if (KIND != KIND_BF16) {
+    const uint32_t desc0 = ti_desc(smem_u32(smem)), sf0 = ti_desc_sf(smem_u32(smem) + C::A_BYTES + C::B_BYTES);
+    bool ok = true;
+    for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
+      const int s = it % ring;
+      if (!mbar_wait_warp(&full_bar[s], (it / ring) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, (int)blockIdx.x); ok = false; break; }
+      if (it == 0 && lane == 0) CL_TRACE(3);
+      tc_fence_after();
+      if (KIND != KIND_BF16) fence_proxy_async_smem();
+      const uint32_t off = (uint32_t)s * (C::STAGE_BYTES / 16), dA = desc0 + off;
+      if (KIND != KIND_BF16) {
 #pragma unroll
-          for (int q = 0; q < C::SF_CHUNKS; ++q) {
-            tc_cp_sf(tmem + L::SFA_COL + 4 * q, umma_desc_sf(sSFA + q * 512));
-            tc_cp_sf(tmem + L::SFB_COL + 4 * q, umma_desc_sf(sSFB + q * 512));
-          }
+        for (int q = 0; q < C::SF_CHUNKS; ++q) {
+          ti_cp_sf(tmem + L::SFA_COL + 4 * q, sf0 + off + q * 32);
+          ti_cp_sf(tmem + L::SFB_COL + 4 * q, sf0 + off + C::SFA_BYTES / 16 + q * 32);
         }
-        const uint64_t adesc = umma_desc_sw128(sA), bdesc = umma_desc_sw128(sB);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const uint32_t accum = (kb > kb0 || k > 0) ? 1u : 0u;
-          if (KIND == KIND_BF16) tc_mma_f16(tmem, adesc + 2 * k, bdesc + 2 * k, make_idesc(KIND_BF16, TN, 0), accum);
-          else if (KIND == KIND_NVFP4)
-            tc_mma_nvf4(tmem, adesc + 2 * k, bdesc + 2 * k, make_idesc(KIND_NVFP4, TN, 0), accum, tmem + L::SFA_COL + 4 * k, tmem + L::SFB_COL + 4 * k);
-          else
-            tc_mma_mxf4(tmem, adesc + 2 * k, bdesc + 2 * k, make_idesc(KIND_MXFP4, TN, (k & 1) * 2), accum, tmem + L::SFA_COL + 4 * (k >> 1),
-                        tmem + L::SFB_COL + 4 * (k >> 1));
-        }
-        tc_commit(&empty_bar[s]);
       }
-      if (ok) tc_commit(&accf_bar);
-      CL_TRACE(4);
+      ti_mma4<C::ISSUE, 4, 4>(tmem, dA, dA + C::A_BYTES / 16, make_idesc(KIND, TN, 0), kb > kb0 ? 1u : 0u, tmem + L::SFA_COL, tmem + L::SFB_COL);
+      ti_commit(&empty_bar[s]);
     }
+    if (ok) ti_commit(&accf_bar);
+    if (lane == 0) CL_TRACE(4);
     __syncwarp();
   } else {
     pdl_wait();

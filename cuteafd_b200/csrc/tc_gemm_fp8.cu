@@ -14,6 +14,7 @@
 // handling of the FP8 backbone (families/deepseek_v4/engine.rs:1320-1390).
 #define CA_PDL_CLASS 1
 #include "tc_gemm_wide.cuh"
+#include "tc_issue.cuh"
 
 enum { F8_EPI_BF16 = 0, F8_EPI_BF16_RESIDUAL = 1, F8_EPI_F32 = 3 };
 
@@ -68,7 +69,7 @@ __global__ void __launch_bounds__(192, (TN <= 32 ? 2 : 1)) fp8_linear_kernel(con
   float* staging = (float*)(smem + ring * C::STAGE_BYTES);                 // [S-1][TN][128] fp32 on cluster rank 0
   float* sc_tab = staging + (size_t)(S - 1 + C::OWN) * 128 * TN;           // [stages of my slice][TN] combined scales
   const bool use_tab = C::table_bytes(nk_max) > 0;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::MAX_RING; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
@@ -132,22 +133,19 @@ __global__ void __launch_bounds__(192, (TN <= 32 ? 2 : 1)) fp8_linear_kernel(con
     }
   } else if (warp == 1) {
     // ---- MMA issuer: one fresh accumulator buffer per stage (= per scale block)
+    // (the whole warp, under an elected lane's predicate: tc_issue.cuh)
     pdl_wait();
-    if (lane == 0) {
-      const uint32_t smem_base = smem_u32(smem);
-      const uint32_t idesc = (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);   // E4M3 x E4M3 -> fp32
-      for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
-        const int s = it % ring, b = it % C::NACC;
-        if (!mbar_wait_bounded(&acce_bar[b], ((it / C::NACC) & 1) ^ 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, (int)blockIdx.x); break; }
-        if (!mbar_wait_bounded(&full_bar[s], (it / ring) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, (int)blockIdx.x); break; }
-        tc_fence_after();
-        const uint32_t st = smem_base + s * C::STAGE_BYTES;
-        const uint64_t adesc = umma_desc_sw128(st), bdesc = umma_desc_sw128(st + C::A_BYTES);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) tc_mma_f8(tmem + b * TN, adesc + 2 * k, bdesc + 2 * k, idesc, k > 0 ? 1u : 0u);
-        tc_commit(&empty_bar[s]);
-        tc_commit(&accf_bar[b]);
-      }
+    const uint32_t desc0 = ti_desc(smem_u32(smem));
+    const uint32_t idesc = (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);   // E4M3 x E4M3 -> fp32
+    for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
+      const int s = it % ring, b = it % C::NACC;
+      if (!mbar_wait_warp(&acce_bar[b], ((it / C::NACC) & 1) ^ 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, (int)blockIdx.x); break; }
+      if (!mbar_wait_warp(&full_bar[s], (it / ring) & 1, abortp)) { ca_dev_fail(a.status, CA_DEV_TIMEOUT_MMA, (int)blockIdx.x); break; }
+      tc_fence_after();
+      const uint32_t dA = desc0 + (uint32_t)s * (C::STAGE_BYTES / 16);
+      ti_mma4<TI_F8>(tmem + b * TN, dA, dA + C::A_BYTES / 16, idesc, 0u);
+      ti_commit(&empty_bar[s]);
+      ti_commit(&accf_bar[b]);
     }
     __syncwarp();
   } else {
