@@ -1,4 +1,4 @@
-// Prompt attention with two query tiles per CTA, for steps with tiles enough to give every SM a pair (rule: `pf_use_pairs`).
+// Prompt attention with two query tiles per CTA, or one where there are too few of them (rule: `pf_tiles_per_cta`).
 //
 // Of one 128-row tile, scores, softmax and P V are a chain: the tensor pipe idles under the softmax and the exponential units under the products
 // (attention_mla_prefill.cu: tensor pipe active 20 to 40 %).  Here a CTA owns two neighbouring tiles A and B of one head; while A's softmax runs,
@@ -12,7 +12,7 @@
 //   threads         warp 0 loads, warp 1 issues, warps 4-7 and 8-11 are A's and B's softmax, one thread per query row
 // Key tiles, the reference maximum's rule and every sum are those of the one-tile kernels: all of a row's values are added key after key, so
 // both give the same bits.
-// Measured, one-tile kernel / this one: 4096 rows of 64 heads over 4: 644 / 303 us; 2048 rows over 8192 keys of 128 latent heads: 1442 / 1126
+// Measured, one-tile kernel / this one: 4096 rows of 64 heads over 4: 643 / 285 us; 2048 rows over 8192 keys of 128 latent heads: 1432 / 1127
 // (a pair takes 3,700 and 4,200 cycles a key tile, 2,048 and 2,560 of them of the tensor pipe; what it waits for is the chain from the last part of P
 // to the next scores).
 #pragma once
@@ -106,7 +106,7 @@ __device__ __forceinline__ void pp_mma_ts(uint32_t d, uint32_t a, uint32_t b_lo,
 #undef PP_TS
 }
 
-template <class Src, int KC, int VC>
+template <class Src, int KC, int VC, int PER_CTA>
 __global__ void __launch_bounds__(PP_THREADS, 1) prefill_pair_kernel(const __grid_constant__ typename Src::Args a) {
   using C = PairCfg<KC, VC>;
   pdl_launch(); pdl_wait();
@@ -127,14 +127,14 @@ __global__ void __launch_bounds__(PP_THREADS, 1) prefill_pair_kernel(const __gri
 
   // the heaviest query tiles (most visible keys) are scheduled first
   const int G = Src::group(a), tok_per_tile = 128 / G;
-  const int head = blockIdx.x, max_pairs = (a.max_q_tiles + 1) / 2;
-  const int seq = blockIdx.y / max_pairs, pair = max_pairs - 1 - blockIdx.y % max_pairs;
+  const int head = blockIdx.x, units = (a.max_q_tiles + PER_CTA - 1) / PER_CTA;
+  const int seq = blockIdx.y / units, unit = units - 1 - blockIdx.y % units;
   const int qlen = a.q_len[seq], kvlen = a.kv_len[seq];
-  const int tok0 = pair * 2 * tok_per_tile;
+  const int tok0 = unit * PER_CTA * tok_per_tile;
   if (tok0 >= qlen) return;
   const bool bidir = Src::bidir(a);
   // tile x: its tokens, and the key tiles that its rows see (0 where there is no such tile)
-  auto tokens_of = [&](int x) { return max(0, min(tok_per_tile, qlen - tok0 - x * tok_per_tile)); };
+  auto tokens_of = [&](int x) { return x >= PER_CTA ? 0 : max(0, min(tok_per_tile, qlen - tok0 - x * tok_per_tile)); };
   auto first_pos_of = [&](int x) { return bidir ? kvlen - 1 : kvlen - qlen + tok0 + x * tok_per_tile; };
   auto tiles_of = [&](int x) {
     const int nt = tokens_of(x);
@@ -388,9 +388,9 @@ __global__ void __launch_bounds__(PP_THREADS, 1) prefill_pair_kernel(const __gri
   if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
-template <class Src, int KC, int VC>
-static int launch_prefill_pair(const typename Src::Args& a, int heads, int n_seq, cudaStream_t s) {
-  auto kern = prefill_pair_kernel<Src, KC, VC>;
+template <class Src, int KC, int VC, int PER_CTA>
+static int launch_prefill_tiles(const typename Src::Args& a, int heads, int n_seq, cudaStream_t s) {
+  auto kern = prefill_pair_kernel<Src, KC, VC, PER_CTA>;
   constexpr int SMEM = PairCfg<KC, VC>::SMEM;
   static bool attr_set[64] = {false};
   int dev = 0; cudaGetDevice(&dev);
@@ -399,6 +399,25 @@ static int launch_prefill_pair(const typename Src::Args& a, int heads, int n_seq
     if (e != cudaSuccess) return ca_cuda(e, "cudaFuncSetAttribute(prefill_pair)");
     attr_set[dev & 63] = true;
   }
-  CA_LAUNCH_PDL(kern, dim3(heads, n_seq * ((a.max_q_tiles + 1) / 2)), PP_THREADS, SMEM, s, a);
+  CA_LAUNCH_PDL(kern, dim3(heads, n_seq * ((a.max_q_tiles + PER_CTA - 1) / PER_CTA)), PP_THREADS, SMEM, s, a);
   return CA_OK;
+}
+// Query tiles per CTA here, or 0: the one-tile kernels.  With keys of up to 128 columns one tile per CTA while that is one wave, else pairs.  us, one-tile
+// kernel / one tile per CTA here / pairs, 64 heads over 4: 296 rows (148 tiles) 24.6 / 16.4 / 20.5; 300 behind 6,000 227 / 178 / 115; 512 40 / 27 / 24;
+// 17 behind 4,000 84 / 66 / 76.
+// Wider keys (192: 12 score products a tile, ring of eight chunks) are slower by themselves than in the one-tile kernel, which keeps the queries in tensor
+// memory: 128 rows behind 4,000 of 128 latent heads 68 / 80, so pairs there have to save waves (a pair takes 1.3 of its steps): 200 behind 4,000
+// 123 / 147 / 100, 257 behind 4,000 180 / 215 / 172, 2048 behind 6,144 1432 / 1588 / 1127.  Less than a wave of pairs only with few
+// tiles, which see about as many keys each (2,048 rows of 16 heads, 1 to 16 key tiles: 47 / 49 / 53).
+static int pf_tiles_per_cta(int kc, int heads, int n_seq, int max_q_tiles) {
+  const long long sms = ca_sm_count(), tiles = (long long)heads * n_seq * max_q_tiles, pairs = (long long)heads * n_seq * ((max_q_tiles + 1) / 2);
+  if (kc <= 2) return tiles <= sms ? 1 : 2;
+  if (pairs < sms && max_q_tiles > 4) return 0;
+  return 4 * ((pairs + sms - 1) / sms) < 3 * ((tiles + sms - 1) / sms) ? 2 : 0;
+}
+template <class Src, int KC, int VC>
+static int launch_prefill_pair(const typename Src::Args& a, int heads, int n_seq, cudaStream_t s) {
+  if constexpr (KC <= 2)
+    if (pf_tiles_per_cta(KC, heads, n_seq, a.max_q_tiles) == 1) return launch_prefill_tiles<Src, KC, VC, 1>(a, heads, n_seq, s);
+  return launch_prefill_tiles<Src, KC, VC, 2>(a, heads, n_seq, s);
 }

@@ -1,5 +1,5 @@
-"""Prompt attention with two query tiles per CTA: steps with tiles enough to take it, against the fp32 oracles of the one-tile kernels' tests, and bit
-for bit against the one-tile kernels (all of a row's values are added in the same order)."""
+"""Prompt attention with one or two query tiles per CTA: steps with tiles enough for two against the fp32 oracles of the one-tile kernels' tests, and both
+bit for bit against the kernel for windows, given one that hides nothing (all of a row's values are added in the same order)."""
 import pytest
 import torch
 
@@ -25,24 +25,26 @@ def test_expanded_against_oracle(H, d, dv, r, gate):
 
 # a lone tile, a ragged pair, a pair whose second tile is one token; over contexts that end inside, at and just behind a key tile
 @pytest.mark.parametrize("q,before", [(8, 0), (9, 119), (16, 112), (17, 240), (300, 0), (130, 1000), (257, 383)])
-def test_paged_same_bits_as_one_tile(q, before):
-    """One sequence by itself leaves most SMs without a pair and takes the one-tile kernel; among enough copies of itself it takes the pairs."""
-    Hq, Hkv, kv, copies = 64, 4, q + before, 40
+@pytest.mark.parametrize("copies", [1, 40])
+def test_paged_same_bits_as_window_kernel(q, before, copies):
+    """One sequence takes a tile per CTA, many copies of it take two; a sliding window as long as the sequence takes the one-tile kernel."""
+    Hq, Hkv, kv = 64, 4, q + before
     g = torch.Generator().manual_seed(q)
     pages = -(-kv // 64)
     cache = torch.randn(1, pages * 64, 2, Hkv, 128, generator=g).to(torch.bfloat16).to(DEV)
     maps, rows = ops.encode_kv_tmaps(cache), (torch.randn(q, Hq * 128, generator=g) * 2).to(torch.bfloat16).to(DEV)
 
-    def run(n):
+    def run(n, window):
         x, out = rows.repeat(n, 1).contiguous(), torch.zeros(n * q, Hq * 128, dtype=torch.bfloat16, device=DEV)
         status, table = torch.zeros(4, dtype=torch.int32, device=DEV), i32([list(range(pages))] * n)
         lens, qs, ql = i32([kv] * n), i32([i * q for i in range(n)]), i32([q] * n)
-        call("cuteafd_gqa_prefill_attention", ptr(x), ptr(maps[0]), ptr(table), ptr(lens), ptr(qs), ptr(ql), None, ptr(out), n * q, n, q, Hq * 128, Hq, Hkv, pages, 0, 128 ** -0.5,
+        call("cuteafd_gqa_prefill_attention", ptr(x), ptr(maps[0]), ptr(table), ptr(lens), ptr(qs), ptr(ql), None, ptr(out), n * q, n, q, Hq * 128, Hq, Hkv, pages, window, 128 ** -0.5,
              ptr(status), stream())
         torch.cuda.synchronize()
         assert int(status[0]) == 0
         return out.view(n, q, -1)
-    alone, many = run(1), run(copies)
-    assert float(alone.float().abs().max()) > 0
+    want, got = run(1, kv), run(copies, 0)
+    assert float(want.float().abs().max()) > 0
     for i in range(copies):
-        assert torch.equal(many[i], alone[0]), i
+        assert torch.equal(got[i], want[0]), i
+
