@@ -20,6 +20,7 @@
 // under them).  With one thread per row a tile's softmax was a single warp's chain per scheduler and bounded the loop:
 // 2048 rows over 8192 keys of 128 heads 1600 us, 1430 now; 4096 rows of 64 heads over 4 (the paged form below) 830 and 640.
 // Every wait is bounded and reports through the status word.
+// Steps with tiles enough for two per CTA take the kernel of attention_prefill_pair.cuh, with the same bits.
 //
 // Reference: the dedicated MLA prefill kernels of the GLM5 family (native/families/glm5/cuda/glm_mla_prefill.cu:123, 539),
 // which also expand the latent cache per chunk and run per-head attention with mma.sync.
