@@ -3,7 +3,9 @@
 // A product's operands (descriptors, tensor-memory addresses, instruction descriptor) are warp-wide registers.  In a branch on the lane number the
 // compiler has to assume that they differ between lanes, and moving them there costs more than the product: 120 to 180 cycles each where a
 // 128 x 128 x 16 bf16 product takes 64.  Here the whole warp runs the issuer's loop, and four products at a time are issued under
-// the elected lane's predicate, their descriptors a constant's distance from the first ones'.
+// the elected lane's predicate, their descriptors a constant's distance from the first ones'.  Branch / this, us per launch: paired prompt attention 435 / 320,
+// FP8 products of a 2,048-row latent prompt 202 / 168, NVFP4 gate + up of 4,096 tokens 330 / 286, of one token 23.5 / 19.8, latent decode attention
+// of 16 sequences at 8k 137 / 114.
 #pragma once
 #include "common.cuh"
 
