@@ -790,7 +790,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) gqa_prefill_kernel(const __grid
 template <int KC, int VC>
 static int launch_gqa_prefill(const GqaPrefillArgs& a, int n_seq, cudaStream_t s) {
   if constexpr (KC <= 3 && VC <= 2)
-    if (a.window <= 0 && pf_tiles_per_cta(KC, a.Hkv, n_seq, a.max_q_tiles)) return launch_prefill_pair<GqaPairSrc, KC, VC>(a, a.Hkv, n_seq, s);
+    if (a.window <= 0 && pf_pair_takes(a.scale) && pf_tiles_per_cta(KC, a.Hkv, n_seq, a.max_q_tiles)) return launch_prefill_pair<GqaPairSrc, KC, VC>(a, a.Hkv, n_seq, s);
   const int smem = GqaPrefillCfg<KC, VC>::SMEM;
   static bool attr_set[64] = {false};
   int dev = 0; cudaGetDevice(&dev);
@@ -884,7 +884,7 @@ extern "C" int cuteafd_latent_gather_ctx(const void* cache, const int* page_tabl
 template <int KN, int KR, int NV>
 static int mla_prefill_launch(const MlaPrefillArgs& a, int n_seq, cudaStream_t s) {
   if constexpr (KN + KR <= 3)
-    if (pf_tiles_per_cta(KN + KR, a.Hl, n_seq, a.max_q_tiles)) return launch_prefill_pair<MlaPairSrc<KN>, KN + KR, NV>(a, a.Hl, n_seq, s);
+    if (pf_pair_takes(a.scale) && pf_tiles_per_cta(KN + KR, a.Hl, n_seq, a.max_q_tiles)) return launch_prefill_pair<MlaPairSrc<KN>, KN + KR, NV>(a, a.Hl, n_seq, s);
   constexpr int SMEM = PF_P_BYTES + PF_NS * (KN + KR) * 16384 + PF_NSV * NV * 16384 + PF_TAIL;
   auto kern = mla_prefill_kernel<KN, KR, NV>;
   static bool attr_set[64] = {false};

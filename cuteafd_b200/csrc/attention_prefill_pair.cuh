@@ -402,6 +402,9 @@ static int launch_prefill_tiles(const typename Src::Args& a, int heads, int n_se
   CA_LAUNCH_PDL(kern, dim3(heads, n_seq * ((a.max_q_tiles + PER_CTA - 1) / PER_CTA)), PP_THREADS, SMEM, s, a);
   return CA_OK;
 }
+// Hidden scores are -inf here before they are scaled, which hides them only if the scale is positive (0 x -inf is NaN): any other takes the one-tile kernels,
+// which clear the probabilities.
+static bool pf_pair_takes(float scale) { return scale > 0.f; }
 // Query tiles per CTA here, or 0: the one-tile kernels.  With keys of up to 128 columns one tile per CTA while that is one wave, else pairs.  us, one-tile
 // kernel / one tile per CTA here / pairs, 64 heads over 4: 296 rows (148 tiles) 24.6 / 16.4 / 20.5; 300 behind 6,000 227 / 178 / 115; 512 40 / 27 / 24;
 // 17 behind 4,000 84 / 66 / 76.
