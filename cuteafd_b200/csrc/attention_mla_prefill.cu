@@ -76,7 +76,7 @@ __device__ __forceinline__ float pf_exp2(float x) { float y; asm("ex2.approx.ftz
 // `xchg` [2][2][128] floats: the halves' maxima of tile i in buffer i & 1; half 0's sum of tile i - 1 travels in half 1's slot of the other buffer,
 // which half 0 has read by then and half 1 writes again only after it read the sum.  `bar` counts both warps' lanes, one phase per tile.
 struct PfRow {
-  float m_ref = -INFINITY, l = 0.f, alpha = 1.f, run = 0.f;
+  float m_ref = -INFINITY, m_sub = 0.f, l = 0.f, alpha = 1.f, run = 0.f;       // m_sub: m_ref, or 0 while no key has scored above -inf (exponentials of -inf)
   float held[PF_KT / 4];
   float* x; uint64_t* bar;
   int hf, r;
@@ -101,7 +101,7 @@ struct PfRow {
     alpha = 1.f;
     if (mx > m_ref + 8.f) {
       if (m_ref != -INFINITY) alpha = exp2f(m_ref - mx);
-      m_ref = mx;
+      m_ref = m_sub = mx;
     }
     return true;
   }
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) mla_prefill_kernel(const __grid
           tc_wait_ld();
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            const float e0 = pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -row.m_ref)), e1 = pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -row.m_ref));
+            const float e0 = pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -row.m_sub)), e1 = pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -row.m_sub));
             row.add(c * 16 + j, e0 + e1);
             bf162 h = __floats2bfloat162_rn(e0, e1);
             pk[c * 16 + j] = *(uint32_t*)&h;
@@ -346,8 +346,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) mla_prefill_kernel(const __grid
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int kp = key0 + hf * 64 + c * 32 + 2 * j;
-            const float e0 = (live && kp <= qpos) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -row.m_ref)) : 0.f;
-            const float e1 = (live && kp + 1 <= qpos) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -row.m_ref)) : 0.f;
+            const float e0 = (live && kp <= qpos) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -row.m_sub)) : 0.f;
+            const float e1 = (live && kp + 1 <= qpos) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -row.m_sub)) : 0.f;
             row.add(c * 16 + j, e0 + e1);
             bf162 h = __floats2bfloat162_rn(e0, e1);
             pk[c * 16 + j] = *(uint32_t*)&h;
@@ -391,7 +391,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) mla_prefill_kernel(const __grid
         const float e1 = (m_nat == -INFINITY) ? 0.f : __expf(m_nat - m2);
         lt = row.l * e1 + __expf(sk - m2); scale_o = e1;
       }
-      const float inv = (lt > 0.f ? scale_o / lt : 0.f) * ((a.gate && live) ? a.gate[(size_t)t * a.Hl + head] : 1.f);      // output gate of the head
+      float inv = (lt > 0.f ? scale_o / lt : 0.f) * ((a.gate && live) ? a.gate[(size_t)t * a.Hl + head] : 1.f);      // output gate of the head
+      if (row.l == 0.f && qpos >= 0 && !a.sink) inv = NAN;                // keys seen, and all of them scored -inf: no weights (a row without keys is 0)
       bf16* dst = a.out + (size_t)t * a.ldo + (size_t)head * a.dv;
       const bool vec = (a.ldo | a.dv) % 8 == 0;
 #pragma unroll 1
@@ -673,7 +674,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) gqa_prefill_kernel(const __grid
           tc_wait_ld();
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            const float e0 = pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -row.m_ref)), e1 = pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -row.m_ref));
+            const float e0 = pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -row.m_sub)), e1 = pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -row.m_sub));
             row.add(c * 16 + j, e0 + e1);
             bf162 h = __floats2bfloat162_rn(e0, e1);
             pk[c * 16 + j] = *(uint32_t*)&h;
@@ -702,8 +703,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) gqa_prefill_kernel(const __grid
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int kp = key0 + hf * 64 + c * 32 + 2 * j;
-            const float e0 = sees(kp) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -row.m_ref)) : 0.f;
-            const float e1 = sees(kp + 1) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -row.m_ref)) : 0.f;
+            const float e0 = sees(kp) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -row.m_sub)) : 0.f;
+            const float e1 = sees(kp + 1) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -row.m_sub)) : 0.f;
             row.add(c * 16 + j, e0 + e1);
             bf162 h = __floats2bfloat162_rn(e0, e1);
             pk[c * 16 + j] = *(uint32_t*)&h;
@@ -749,7 +750,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) gqa_prefill_kernel(const __grid
         const float e1 = (m_nat == -INFINITY) ? 0.f : __expf(m_nat - m2);
         lt = row.l * e1 + __expf(sk - m2); scale_o = e1;
       }
-      const float inv = (lt > 0.f ? scale_o / lt : 0.f) * a.x.head_factor(t, h);
+      float inv = (lt > 0.f ? scale_o / lt : 0.f) * a.x.head_factor(t, h);
+      if (row.l == 0.f && qpos >= 0 && !a.x.sink) inv = NAN;              // as above
       const bool gated = a.x.gate && a.x.gate_values;
       bf16* dst = a.out + (size_t)t * a.ldo + (size_t)h * a.dv;
       const bool vec = ((a.dv | a.ldo) & 7) == 0;

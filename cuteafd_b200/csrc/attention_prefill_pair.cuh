@@ -349,7 +349,8 @@ __global__ void __launch_bounds__(PP_THREADS, 1) prefill_pair_kernel(const __gri
         const float e1 = (m_nat == -INFINITY) ? 0.f : __expf(m_nat - m2);
         lt = l * e1 + __expf(sk - m2); scale_o = e1;
       }
-      const float inv = (lt > 0.f ? scale_o / lt : 0.f) * (live ? Src::head_factor(a, t, h) : 1.f);
+      float inv = (lt > 0.f ? scale_o / lt : 0.f) * (live ? Src::head_factor(a, t, h) : 1.f);
+      if (l == 0.f && qpos >= 0 && !Src::sink(a)) inv = NAN;          // keys seen, and all of them scored -inf: no weights (a row without keys is 0)
       const bool gated = Src::gated(a);
       bf16* dst = a.out + (size_t)t * a.ldo + (size_t)h * a.dv;
       const bool vec = ((a.dv | a.ldo) & 7) == 0;

@@ -167,3 +167,27 @@ def test_scales_that_are_not_positive(form, scale):
     for i in range(len(seqs)):
         want = step.want(i, scale, True) if bidir else step.want(i, scale)
         assert close(got[step.rows(i)], want), (i, float((got[step.rows(i)].double() - want).abs().max()))
+
+
+@pytest.mark.parametrize("form", ["one tile", "pairs", "bidirectional", "window", "latent", "latent pairs", "wide latent"])
+def test_rows_whose_keys_all_score_minus_infinity_are_nan(form):
+    """As a softmax over nothing else is; rows that see one more key, or none of these, are not."""
+    seqs, low = [(300, 0), (64, 200), (17, 0)], [(0, 150), (0, 130), (0, 1)]
+    if "latent" in form:
+        step = LatentStep(seqs, *{"latent": (3, 1, 1, 2), "latent pairs": (48, 2, 1, 2), "wide latent": (3, 3, 1, 2)}[form])
+        step.q[..., 0] = 1
+        for at, (lo, hi) in zip(step.ctx, low):
+            step.kvb[at + lo:at + hi, :, 0] = -float("inf")
+    else:
+        step = PagedStep(seqs, *((8, 8) if form == "one tile" else (128, 16)))
+        step.q[..., 0] = 1
+        for k, slots, (lo, hi) in zip(step.k, step.slots, low):
+            k[lo:hi, :, 0] = -float("inf")
+            step.store[slots[lo:hi, None], torch.arange(step.Hkv, device=DEV) * 128] = -float("inf")
+    bidir = form == "bidirectional"
+    got = step.run(0.1, -1) if bidir else step.run(0.1, 300) if form == "window" else step.run(0.1)
+    for i in range(len(seqs)):
+        want = step.want(i, 0.1, True) if bidir else step.want(i, 0.1)
+        out, none = got[step.rows(i)], want.isnan()
+        assert bool(none.any()) == (not bidir and i != 1) and torch.equal(out.isnan(), none)
+        assert close(out[~none], want[~none])
