@@ -20,7 +20,7 @@
 // under them).  With one thread per row a tile's softmax was a single warp's chain per scheduler and bounded the loop:
 // 2048 rows over 8192 keys of 128 heads 1600 us, 1430 now; 4096 rows of 64 heads over 4 (the paged form below) 830 and 640.
 // Every wait is bounded and reports through the status word.
-// Steps with tiles enough for two per CTA take the kernel of attention_prefill_pair.cuh, with the same bits.
+// Which steps take the kernel of attention_prefill_pair.cuh instead, with the same bits: `pf_tiles_paged` and `pf_tiles_latent` there.
 //
 // Reference: the dedicated MLA prefill kernels of the GLM5 family (native/families/glm5/cuda/glm_mla_prefill.cu:123, 539),
 // which also expand the latent cache per chunk and run per-head attention with mma.sync.
@@ -792,7 +792,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) gqa_prefill_kernel(const __grid
 template <int KC, int VC>
 static int launch_gqa_prefill(const GqaPrefillArgs& a, int n_seq, cudaStream_t s) {
   if constexpr (KC <= 3 && VC <= 2)
-    if (a.window <= 0 && pf_pair_takes(a.scale) && pf_tiles_per_cta(KC, a.Hkv, n_seq, a.max_q_tiles)) return launch_prefill_pair<GqaPairSrc, KC, VC>(a, a.Hkv, n_seq, s);
+    if (a.window <= 0 && pf_pair_takes(a.scale))
+      if (const int per_cta = pf_tiles_paged(KC, a.Hkv, n_seq, a.max_q_tiles)) return launch_prefill_pair<GqaPairSrc, KC, VC>(a, a.Hkv, n_seq, per_cta, s);
   const int smem = GqaPrefillCfg<KC, VC>::SMEM;
   static bool attr_set[64] = {false};
   int dev = 0; cudaGetDevice(&dev);
@@ -884,9 +885,10 @@ extern "C" int cuteafd_latent_gather_ctx(const void* cache, const int* page_tabl
 }
 
 template <int KN, int KR, int NV>
-static int mla_prefill_launch(const MlaPrefillArgs& a, int n_seq, cudaStream_t s) {
+static int mla_prefill_launch(const MlaPrefillArgs& a, int n_seq, int max_q_len, cudaStream_t s) {
   if constexpr (KN + KR <= 3)
-    if (pf_pair_takes(a.scale) && pf_tiles_per_cta(KN + KR, a.Hl, n_seq, a.max_q_tiles)) return launch_prefill_pair<MlaPairSrc<KN>, KN + KR, NV>(a, a.Hl, n_seq, s);
+    if (pf_pair_takes(a.scale))
+      if (const int per_cta = pf_tiles_latent(KN, KR, NV, a.Hl, n_seq, a.T, max_q_len)) return launch_prefill_pair<MlaPairSrc<KN>, KN + KR, NV>(a, a.Hl, n_seq, per_cta, s);
   constexpr int SMEM = PF_P_BYTES + PF_NS * (KN + KR) * 16384 + PF_NSV * NV * 16384 + PF_TAIL;
   auto kern = mla_prefill_kernel<KN, KR, NV>;
   static bool attr_set[64] = {false};
@@ -916,7 +918,7 @@ extern "C" int cuteafd_mla_prefill_attention(const void* q_nope, const void* q_r
   a.q_nope = (const bf16*)q_nope; a.q_rope = (const bf16*)q_rope; a.ctx_start = ctx_start; a.kv_len = kv_len; a.q_start = q_start; a.q_len = q_len;
   a.out = (bf16*)out; a.status = status; a.T = T; a.Hl = Hl; a.max_q_tiles = (max_q_len + 127) / 128; a.scale = scale;
   a.gate = nullptr; a.ldt = T; a.ldo = Hl * 128; a.dv = 128; a.sink = nullptr; a.qr_t = Hl * 64; a.qr_h = 64; a.rope_col = 512;
-  rc = mla_prefill_launch<2, 1, 2>(a, n_seq, s);
+  rc = mla_prefill_launch<2, 1, 2>(a, n_seq, max_q_len, s);
   if (rc) return rc;
   CA_CHECK_LAUNCH("mla_prefill_attention");
   return CA_OK;
@@ -950,7 +952,7 @@ extern "C" int cuteafd_latent_prefill_attention(const void* q, const void* q_rop
   a.q_nope = (const bf16*)q; a.q_rope = (const bf16*)q_rope; a.ctx_start = ctx_start; a.kv_len = kv_len; a.q_start = q_start; a.q_len = q_len;
   a.gate = gate; a.out = (bf16*)out; a.status = status; a.T = T; a.Hl = Hl; a.max_q_tiles = (max_q_len + 127) / 128; a.scale = scale;
   a.ldt = ldt; a.ldo = ldo; a.dv = dv;
-#define LP_CASE(K_, R_, V_) if (dk_pad == K_ * 64 && dv_pad == V_ * 64 && (q_rope != nullptr) == (R_ != 0)) rc = mla_prefill_launch<K_, R_, V_>(a, n_seq, s);
+#define LP_CASE(K_, R_, V_) if (dk_pad == K_ * 64 && dv_pad == V_ * 64 && (q_rope != nullptr) == (R_ != 0)) rc = mla_prefill_launch<K_, R_, V_>(a, n_seq, max_q_len, s);
 #define LP_ROW(R_, V_) LP_CASE(1, R_, V_) LP_CASE(2, R_, V_) LP_CASE(3, R_, V_)
   LP_ROW(0, 1) LP_ROW(0, 2) LP_ROW(1, 1) LP_ROW(1, 2)
   if (rc) return rc;

@@ -1,4 +1,4 @@
-// Prompt attention with two query tiles per CTA, or one where there are too few of them (rule: `pf_tiles_per_cta`).
+// Prompt attention with two query tiles per CTA, or one where there are too few of them (rules: `pf_tiles_paged`, `pf_tiles_latent`).
 //
 // Of one 128-row tile, scores, softmax and P V are a chain: the tensor pipe idles under the softmax and the exponential units under the products
 // (attention_mla_prefill.cu: tensor pipe active 20 to 40 %).  Here a CTA owns two neighbouring tiles A and B of one head; while A's softmax runs,
@@ -35,6 +35,7 @@ struct PairCfg {
 // What differs between the paged and the expanded form: where a tile's rows, keys and values lie.
 struct GqaPairSrc {
   using Args = GqaPrefillArgs;
+  template <int KC, int VC> static constexpr bool alone() { return KC <= 2; }           // whether the rules below give such steps one tile per CTA
   static __device__ __forceinline__ int group(const Args& a) { return a.Hq / a.Hkv; }
   static __device__ __forceinline__ bool bidir(const Args& a) { return a.window < 0; }
   template <int KC>
@@ -61,6 +62,7 @@ struct GqaPairSrc {
 template <int KN>
 struct MlaPairSrc {
   using Args = MlaPrefillArgs;
+  template <int KC, int VC> static constexpr bool alone() { return KC == KN && KN + VC <= 3; }
   static __device__ __forceinline__ int group(const Args&) { return 1; }
   static __device__ __forceinline__ bool bidir(const Args&) { return false; }
   template <int KC>
@@ -406,22 +408,50 @@ static int launch_prefill_tiles(const typename Src::Args& a, int heads, int n_se
 // Hidden scores are -inf here before they are scaled, which hides them only if the scale is positive (0 x -inf is NaN): any other takes the one-tile kernels,
 // which clear the probabilities.
 static bool pf_pair_takes(float scale) { return scale > 0.f; }
-// Query tiles per CTA here, or 0: the one-tile kernels.  With keys of up to 128 columns one tile per CTA while that is one wave, else pairs.  us, one-tile
-// kernel / one tile per CTA here / pairs, 64 heads over 4: 296 rows (148 tiles) 24.6 / 16.4 / 20.5; 300 behind 6,000 227 / 178 / 115; 512 40 / 27 / 24;
-// 17 behind 4,000 84 / 66 / 76.
-// Wider keys (192: 12 score products a tile, ring of eight chunks) are slower by themselves than in the one-tile kernel, which keeps the queries in tensor
-// memory: 128 rows behind 4,000 of 128 latent heads 68 / 80, so pairs there have to save waves (a pair takes 1.3 of its steps): 200 behind 4,000
-// 123 / 147 / 100, 257 behind 4,000 180 / 215 / 172, 2048 behind 6,144 1432 / 1588 / 1127.  Less than a wave of pairs only with few
-// tiles, which see about as many keys each (2,048 rows of 16 heads, 1 to 16 key tiles: 47 / 49 / 53).
-static int pf_tiles_per_cta(int kc, int heads, int n_seq, int max_q_tiles) {
-  const long long sms = ca_sm_count(), tiles = (long long)heads * n_seq * max_q_tiles, pairs = (long long)heads * n_seq * ((max_q_tiles + 1) / 2);
-  if (kc <= 2) return tiles <= sms ? 1 : 2;
-  if (pairs < sms && max_q_tiles > 4) return 0;
-  return 4 * ((pairs + sms - 1) / sms) < 3 * ((tiles + sms - 1) / sms) ? 2 : 0;
+// Query tiles per CTA here, or 0: the one-tile kernels.
+//
+// A pair takes 1.3 to 1.6 of a tile's time, so pairs have to save whole waves; less than a wave of them pays only with few tiles, which see about as many keys each
+// (2,048 rows of 16 latent heads, 1 to 16 key tiles, one-tile kernel / pairs: 59 / 70 us).
+static bool pf_pairs_save_waves(long long tiles, long long pairs, int max_q_tiles) {
+  const long long sms = ca_sm_count();
+  return (pairs >= sms || max_q_tiles <= 4) && 4 * ((pairs + sms - 1) / sms) < 3 * ((tiles + sms - 1) / sms);
+}
+// Paged: with keys of up to 128 columns one tile per CTA while that is one wave, else pairs.  us, one-tile kernel / one tile per CTA here / pairs, 64 heads over 4:
+// 296 rows (148 tiles) 24.6 / 16.4 / 20.5; 300 behind 6,000 227 / 178 / 115; 512 40 / 27 / 24; 17 behind 4,000 84 / 66 / 76.
+// In 400 random steps (1 to 49 sequences, 1 to 32 key heads, keys of 64 to 192 and values of 64 and 128 columns) no choice of this rule is slower than the one-tile kernel.
+static int pf_tiles_paged(int kc, int heads, int n_seq, int max_q_tiles) {
+  const long long tiles = (long long)heads * n_seq * max_q_tiles, pairs = (long long)heads * n_seq * ((max_q_tiles + 1) / 2);
+  if (kc <= 2) return tiles <= ca_sm_count() ? 1 : 2;
+  return pf_pairs_save_waves(tiles, pairs, max_q_tiles) ? 2 : 0;
+}
+// Latent: the one-tile kernel takes less per tile than the paged one, so a lone tile here gains little or loses.  One-tile kernel / one tile per CTA here / pairs, us
+// (columns of keys, rotated ones behind the +, and of values; rows, behind as many): 64 and 64, 2,048 rows of 12 heads 36 / 34 / 40; 128 and 128, 64 behind 4,000 of 48 heads
+// 58 / 67 / 65; 64 + 64 and 128, 2,048 of 12 heads 38 / 44 / 50; 128 + 64 and 128, 128 heads, 200 behind 4,000 125 / - / 101, 257 behind 4,000 183 / - / 177, 2,048 behind
+// 6,144 1473 / - / 1178.  On average over random steps of lone tiles, one tile per CTA here takes 0.88 to 1.02 of the one-tile kernel's time with up to 192 columns of keys and
+// values and no rotated ones, 0.95 to 1.09 with 128 and 128, 1.08 to 1.18 with 64 + 64, and pairs' lone tiles 0.9 to 1.2 with 192.
+// Of sequences of different lengths the grid's rectangle says little; `T` bounds how many tiles and pairs there are.  What pairs win is won by second tiles, what they
+// lose is lost by lone ones: 128 + 64 and 128, 16 heads, 1,024 rows beside 15 of one behind 4,000 142 / - / 155; 64 heads, 2,048 behind 4,000 beside 20 of one behind 500
+// 824 / - / 647.  Contexts are on the device, so lone tiles that read far more keys than the prompts do lose all the same (128 heads, the first of these: 890 / - / 1011).
+// Where the lines lie: of 5,000 random steps (1 to 49 sequences, 2 to 128 heads, all widths) 2.4 % are over 4 % slower than in the one-tile kernel, with the rule of the paged form 19 %.
+static int pf_tiles_latent(int kn, int kr, int vc, int heads, int n_seq, int T, int max_q_len) {
+  const long long max_q_tiles = (max_q_len + 127) / 128;
+  long long tiles = n_seq * max_q_tiles, pairs = n_seq * ((max_q_tiles + 1) / 2);
+  bool two;
+  if (T >= (long long)n_seq * max_q_len) two = pf_pairs_save_waves(heads * tiles, heads * pairs, (int)max_q_tiles);
+  else {
+    tiles = heads * min(tiles, (T + n_seq * 127LL) / 128); pairs = heads * min(pairs, (T + n_seq * 255LL) / 256);
+    const long long second = tiles - pairs, lone = pairs - second;
+    two = 20 * second > 15 * ca_sm_count() + lone;
+  }
+  return two ? 2 : kr == 0 && kn + vc <= 3 ? 1 : 0;
 }
 template <class Src, int KC, int VC>
-static int launch_prefill_pair(const typename Src::Args& a, int heads, int n_seq, cudaStream_t s) {
-  if constexpr (KC <= 2)
-    if (pf_tiles_per_cta(KC, heads, n_seq, a.max_q_tiles) == 1) return launch_prefill_tiles<Src, KC, VC, 1>(a, heads, n_seq, s);
+static int launch_prefill_pair(const typename Src::Args& a, int heads, int n_seq, int per_cta, cudaStream_t s) {
+  if constexpr (Src::template alone<KC, VC>())
+    if (per_cta == 1) return launch_prefill_tiles<Src, KC, VC, 1>(a, heads, n_seq, s);
   return launch_prefill_tiles<Src, KC, VC, 2>(a, heads, n_seq, s);
+}
+// The latent rule's answer, for tests; widths in chunks of 64 columns.
+extern "C" int cuteafd_latent_prefill_tiles(int key_chunks, int rotated_chunks, int value_chunks, int heads, int n_seq, int T, int max_q_len) {
+  return pf_tiles_latent(key_chunks, rotated_chunks, value_chunks, heads, n_seq, T, max_q_len);
 }

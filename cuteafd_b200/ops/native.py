@@ -106,6 +106,7 @@ _PROTOS = {
     "cuteafd_latent_attention": [P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, P, P],
     "cuteafd_tmap_encode_latent_rows": [P, P, U64, U64, U64],
     "cuteafd_latent_prefill_attention": [P, P, P, P, I, I, P, L, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, P, P],
+    "cuteafd_latent_prefill_tiles": [I, I, I, I, I, I, I],
     "cuteafd_latent_gather_ctx": [P, P, P, P, P, I, I, I, L, L, I, I, P, P],
     "cuteafd_latent_attention_simt": [P, P, I, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, I, P, P],
     "cuteafd_latent_prepare": [P, I, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, F, I, P, P],
