@@ -24,6 +24,7 @@
 //
 // Reference: the dedicated MLA prefill kernels of the GLM5 family (native/families/glm5/cuda/glm_mla_prefill.cu:123, 539),
 // which also expand the latent cache per chunk and run per-head attention with mma.sync.
+#include <float.h>
 #include <string.h>
 
 #define CA_PDL_CLASS 2
@@ -38,6 +39,7 @@
 #define PF_TAIL 2304              // barriers (256 bytes), what the two threads of a row exchange (2 x 2 x 128 floats)
 #define PF_P_BYTES 32768          // 2 chunks (64 keys each) x [128 rows x 128 B]
 #define PF_V_STAGE 32768          // 2 chunks (64 dims each) x [128 keys x 128 B]
+#define PF_NONE (-FLT_MAX)        // reference maximum of a row no key of which has scored above -inf yet: finite, so that such scores are exponentials of -inf
 
 struct MlaPrefillArgs {
   const bf16* q_nope;           // [Hl, T, 128] head-major
@@ -76,7 +78,7 @@ __device__ __forceinline__ float pf_exp2(float x) { float y; asm("ex2.approx.ftz
 // `xchg` [2][2][128] floats: the halves' maxima of tile i in buffer i & 1; half 0's sum of tile i - 1 travels in half 1's slot of the other buffer,
 // which half 0 has read by then and half 1 writes again only after it read the sum.  `bar` counts both warps' lanes, one phase per tile.
 struct PfRow {
-  float m_ref = -INFINITY, m_sub = 0.f, l = 0.f, alpha = 1.f, run = 0.f;       // m_sub: m_ref, or 0 while no key has scored above -inf (exponentials of -inf)
+  float m_ref = PF_NONE, l = 0.f, alpha = 1.f, run = 0.f;
   float held[PF_KT / 4];
   float* x; uint64_t* bar;
   int hf, r;
@@ -100,8 +102,8 @@ struct PfRow {
     mx = fmaxf(mx, xi[(hf ^ 1) * 128 + r]);
     alpha = 1.f;
     if (mx > m_ref + 8.f) {
-      if (m_ref != -INFINITY) alpha = exp2f(m_ref - mx);
-      m_ref = m_sub = mx;
+      if (m_ref != PF_NONE) alpha = exp2f(m_ref - mx);
+      m_ref = mx;
     }
     return true;
   }
@@ -317,7 +319,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) mla_prefill_kernel(const __grid
           tc_wait_ld();
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            const float e0 = pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -row.m_sub)), e1 = pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -row.m_sub));
+            const float e0 = pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -row.m_ref)), e1 = pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -row.m_ref));
             row.add(c * 16 + j, e0 + e1);
             bf162 h = __floats2bfloat162_rn(e0, e1);
             pk[c * 16 + j] = *(uint32_t*)&h;
@@ -346,8 +348,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) mla_prefill_kernel(const __grid
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int kp = key0 + hf * 64 + c * 32 + 2 * j;
-            const float e0 = (live && kp <= qpos) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -row.m_sub)) : 0.f;
-            const float e1 = (live && kp + 1 <= qpos) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -row.m_sub)) : 0.f;
+            const float e0 = (live && kp <= qpos) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -row.m_ref)) : 0.f;
+            const float e1 = (live && kp + 1 <= qpos) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -row.m_ref)) : 0.f;
             row.add(c * 16 + j, e0 + e1);
             bf162 h = __floats2bfloat162_rn(e0, e1);
             pk[c * 16 + j] = *(uint32_t*)&h;
@@ -387,7 +389,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) mla_prefill_kernel(const __grid
       const int t = row_base + (live ? r : 0);
       float scale_o = 1.f, lt = row.l;
       if (a.sink) {                                     // learned sink logit: one more softmax term with a zero value
-        const float m_nat = (row.m_ref == -INFINITY) ? -INFINITY : row.m_ref * 0.6931471805599453f, sk = a.sink[head], m2 = fmaxf(m_nat, sk);
+        const float m_nat = (row.m_ref == PF_NONE) ? -INFINITY : row.m_ref * 0.6931471805599453f, sk = a.sink[head], m2 = fmaxf(m_nat, sk);
         const float e1 = (m_nat == -INFINITY) ? 0.f : __expf(m_nat - m2);
         lt = row.l * e1 + __expf(sk - m2); scale_o = e1;
       }
@@ -674,7 +676,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) gqa_prefill_kernel(const __grid
           tc_wait_ld();
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            const float e0 = pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -row.m_sub)), e1 = pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -row.m_sub));
+            const float e0 = pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -row.m_ref)), e1 = pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -row.m_ref));
             row.add(c * 16 + j, e0 + e1);
             bf162 h = __floats2bfloat162_rn(e0, e1);
             pk[c * 16 + j] = *(uint32_t*)&h;
@@ -703,8 +705,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) gqa_prefill_kernel(const __grid
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int kp = key0 + hf * 64 + c * 32 + 2 * j;
-            const float e0 = sees(kp) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -row.m_sub)) : 0.f;
-            const float e1 = sees(kp + 1) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -row.m_sub)) : 0.f;
+            const float e0 = sees(kp) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j]), sc2, -row.m_ref)) : 0.f;
+            const float e1 = sees(kp + 1) ? pf_exp2(fmaf(__uint_as_float(sr[2 * j + 1]), sc2, -row.m_ref)) : 0.f;
             row.add(c * 16 + j, e0 + e1);
             bf162 h = __floats2bfloat162_rn(e0, e1);
             pk[c * 16 + j] = *(uint32_t*)&h;
@@ -745,7 +747,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) gqa_prefill_kernel(const __grid
       const int t = row_base + rr / G, h = kvh * G + rr % G;
       float scale_o = 1.f, lt = row.l;
       if (a.x.sink) {                                   // learned sink logit: one more softmax term with a zero value
-        const float m_nat = (row.m_ref == -INFINITY) ? -INFINITY : row.m_ref * 0.6931471805599453f;
+        const float m_nat = (row.m_ref == PF_NONE) ? -INFINITY : row.m_ref * 0.6931471805599453f;
         const float sk = a.x.sink[h], m2 = fmaxf(m_nat, sk);
         const float e1 = (m_nat == -INFINITY) ? 0.f : __expf(m_nat - m2);
         lt = row.l * e1 + __expf(sk - m2); scale_o = e1;
