@@ -1049,6 +1049,8 @@ extern "C" int cuteafd_tc_linear(int kind, int swiglu, int tn, const void* tmA, 
       return ca_gemm_wide(kind, swiglu != 0, wa, items, stream);
     }
   }
+  const int stage_k = kind == KIND_BF16 ? 64 : kind == KIND_W4A8 ? 128 : 256;
+  a.splits = min(a.splits, max(1, (K + stage_k - 1) / stage_k));       // a part without a stage has no product, and the fix-up would add what its tensor memory held before
   long long work = tiles ? (long long)max_tiles * n_nt : (long long)((rows_total + tn - 1) / tn) * n_nt * a.splits;
   int cap = max_ctas > 0 ? max_ctas : ca_sm_count() * (tn <= 32 ? 2 : 1);
   int grid = (int)(work < cap ? work : cap);

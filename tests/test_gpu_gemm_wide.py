@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from cuteafd_b200 import ops
-from cuteafd_b200.ops import ActBuffer, TcWeight, KIND_BF16, KIND_FP8B, KIND_MXFP4, KIND_NVFP4
+from cuteafd_b200.ops import ActBuffer, TcWeight, KIND_BF16, KIND_FP8B, KIND_MXFP4, KIND_NVFP4, KIND_W4A8
 from cuteafd_b200.ref import quant
 
 pytestmark = pytest.mark.gpu
@@ -137,3 +137,18 @@ def test_more_parts_than_stages():
     torch.cuda.synchronize()
     ref = x.double() @ w.dequantize()[0].double().to(DEV).T
     assert int(st[0]) == 0 and float((y.double() - ref).norm() / ref.norm()) < 1e-6 * 192 ** 0.5
+
+
+@pytest.mark.parametrize("kind,tn,K", [(KIND_BF16, 32, 192), (KIND_BF16, 64, 128), (KIND_BF16, 256, 320), (KIND_NVFP4, 64, 512), (KIND_MXFP4, 256, 768), (KIND_W4A8, 64, 256), (KIND_W4A8, 128, 640)])
+def test_more_parts_than_stages_in_narrow_tiles(kind, tn, K):
+    """The same through the fix-up over CTAs, whose empty parts must not add what an earlier product left in tensor memory."""
+    rows = min(tn, 200)
+    w, st = TcWeight.random(1, 320, K, kind, DEV, seed=3), torch.zeros(4, dtype=torch.int32, device=DEV)
+    x = torch.randn(rows, K, device=DEV).to(torch.bfloat16)
+    act, loud, whole, parts = operand(kind, x, tn), operand(kind, x * 50, tn), torch.zeros(rows, 320, device=DEV), torch.zeros(rows, 320, device=DEV)
+    ops.tc_linear(w, act, whole, status=st)
+    for _ in range(3):
+        ops.tc_linear(w, loud, parts, status=st)
+        ops.tc_linear(w, act, parts, splits=8, status=st)
+        torch.cuda.synchronize()
+        assert int(st[0]) == 0 and float((parts - whole).norm() / whole.norm()) < 1e-6 * K ** 0.5       # fp32 sums of K products in another order
