@@ -1,10 +1,11 @@
-"""Prompt attention with one or two query tiles per CTA: steps with tiles enough for two against the fp32 oracles of the one-tile kernels' tests, and both
-bit for bit against the kernel for windows, given one that hides nothing (all of a row's values are added in the same order)."""
+"""Prompt attention with one or two query tiles per CTA: steps with tiles enough for two against the fp32 oracles of the one-tile kernels' tests, both
+bit for bit against the kernel for windows, given one that hides nothing (all of a row's values are added in the same order), and every width and mask against a
+softmax in 64 bits."""
 import pytest
 import torch
 
 from cuteafd_b200 import ops
-from cuteafd_b200.ops.native import call, ptr, stream
+from cuteafd_b200.ops.native import call, lib, ptr, stream
 from test_gpu_kernels import test_gqa_prefill_attention as check_gqa
 from test_gpu_latent_stack import test_expanding_prefill_attention as check_latent
 
@@ -191,3 +192,45 @@ def test_rows_whose_keys_all_score_minus_infinity_are_nan(form):
         out, none = got[step.rows(i)], want.isnan()
         assert bool(none.any()) == (not bidir and i != 1) and torch.equal(out.isnan(), none)
         assert close(out[~none], want[~none])
+
+
+# contexts of more than eight key tiles: with 192 columns of keys and 128 of values the ring's eight chunks go round every 1.6 of them
+LATENT = [(kn, kr, nv) for kr in (0, 1) for kn in (1, 2, 3) if kn + kr <= 3 for nv in (1, 2)]
+
+
+@pytest.mark.parametrize("kn,kr,nv", LATENT)
+def test_latent_pairs(kn, kr, nv):
+    """Against the 64-bit softmax, and bit for bit what few heads give, which take one tile per CTA here or the one-tile kernel."""
+    seqs, H, scale = [(250, 900), (257, 383), (20, 1300)], 64, 0.7 * ((kn + kr) * 64) ** -0.5
+    step, tiles = LatentStep(seqs, H, kn, kr, nv), lib().cuteafd_latent_prefill_tiles
+    assert tiles(kn, kr, nv, H, step.n, step.T, step.max_q) == 2 and tiles(kn, kr, nv, 2, step.n, step.T, step.max_q) < 2
+    got = step.run(scale)
+    for heads in ([0, 41], [63]):
+        assert torch.equal(got[:, heads], step.run(scale, heads))
+    for i in range(len(seqs)):
+        assert close(got[step.rows(i)], step.want(i, scale))
+
+
+@pytest.mark.parametrize("heads", [(4, 4), (16, 2), (64, 64), (128, 16)])
+def test_bidirectional_sequences_of_unequal_lengths(heads):
+    """The first two: one tile per CTA; the others: pairs."""
+    step = PagedStep([(300, 0), (129, 0), (100, 60), (17, 0), (256, 0), (1, 0)], *heads)
+    got = step.run(0.06, -1)
+    for i in range(step.n):
+        assert close(got[step.rows(i)], step.want(i, 0.06, True))
+
+
+@pytest.mark.parametrize("heads", [(6, 2), (160, 80)])
+@pytest.mark.parametrize("dk,dv", [(64, 64), (40, 128), (128, 24), (100, 65), (192, 64), (160, 128)])
+@pytest.mark.parametrize("gate", ["head", "value", None])
+def test_sinks_gates_and_factors_without_a_window(heads, dk, dv, gate):
+    """Few heads: one tile per CTA (with 192 columns of keys: the one-tile kernel); many: pairs."""
+    (Hq, Hkv), scale = heads, 1.3 * dk ** -0.5
+    step = PagedStep([(250, 0), (250, 640)], Hq, Hkv, dk, dv)
+    sink, logits = torch.randn(Hq, generator=step.gen, device=DEV) + 2, step.randn(step.T, 3 + Hq * dv)[:, 3:]
+    x = ops.attn_extras(sink=sink, gate=None if gate is None else logits, per_value=gate == "value", out_scale=0.6)
+    got = step.run(scale, 0, x)
+    for i in range(step.n):
+        g = logits[step.rows(i)].double().sigmoid()
+        factor = {"head": lambda: g[:, :Hq, None], "value": lambda: g.view(-1, Hq, dv), None: lambda: 1.0}[gate]()
+        assert close(got[step.rows(i)], step.want(i, scale, sink=sink) * factor * 0.6)

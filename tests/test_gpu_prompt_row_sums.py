@@ -1,4 +1,4 @@
-"""The order in which prompt attention adds up a row's probabilities: key after key, tile after tile, although two threads share a row.  Layers
+"""The order in which prompt attention adds up a row's probabilities: key after key, tile after tile, also where two threads share a row.  Layers
 behind it choose experts and quantise from these bits."""
 import numpy as np
 import pytest
@@ -30,7 +30,7 @@ def row(n_tiles: int, at: int):
 
 
 @pytest.mark.parametrize("n_tiles,at", [(1, 0), (2, 0), (2, 1), (3, 1), (4, 3)])
-@pytest.mark.parametrize("form", ["paged", "latent"])
+@pytest.mark.parametrize("form", ["paged", "window", "latent"])
 def test_row_sum_is_taken_key_after_key(form, n_tiles, at):
     score, value = row(n_tiles, at)
     n = n_tiles * TILE
@@ -39,12 +39,12 @@ def test_row_sum_is_taken_key_after_key(form, n_tiles, at):
     q = torch.zeros(1, 128, dtype=torch.bfloat16, device=DEV)
     q[0, 0] = 1
     kv_len, q_start, q_len = i32([n]), i32([0]), i32([1])
-    if form == "paged":
+    if form != "latent":                                                 # without a window one thread has the row, with one two share it, as in the latent form
         kv = torch.zeros(1, n, 2, 1, 128, dtype=torch.bfloat16, device=DEV)
         kv[0, :, 0, 0, 0], kv[0, :, 1, 0] = score.to(DEV), value[:, None].to(DEV)
         maps, table = ops.encode_kv_tmaps(kv), i32([list(range(n // 64))])
         call("cuteafd_gqa_prefill_attention", ptr(q), ptr(maps[0]), ptr(table), ptr(kv_len), ptr(q_start), ptr(q_len), None, ptr(out), 1, 1, 1, 128, 1, 1,
-             table.shape[1], 0, unit_scale(), ptr(st), stream())
+             table.shape[1], n if form == "window" else 0, unit_scale(), ptr(st), stream())
     else:
         kvb = torch.zeros(n + 64, 256, dtype=torch.bfloat16, device=DEV)
         kvb[:n, 0], kvb[:n, 128:] = score.to(DEV), value[:, None].to(DEV)
