@@ -50,7 +50,6 @@ struct MlaArgs {
   float scale;
 };
 
-__device__ __forceinline__ uint64_t mla_desc_k_sw128(uint32_t saddr) { return umma_desc_sw128(saddr); }
 __device__ __forceinline__ uint64_t mla_desc_mn_sw128(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
   return (uint64_t)((saddr & 0x3FFFF) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }

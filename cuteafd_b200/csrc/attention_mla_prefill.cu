@@ -34,11 +34,9 @@
 #define PF_KT 128                 // keys per tile
 #define PF_NS 2                   // K stages
 #define PF_NSV 2                  // V stages
-#define PF_Q_BYTES 0              // the query tile lives in tensor memory (A operand of the score MMAs)
 #define PF_THREADS 320            // producer, MMA issuer, 2 x 4 softmax warps
 #define PF_TAIL 2304              // barriers (256 bytes), what the two threads of a row exchange (2 x 2 x 128 floats)
 #define PF_P_BYTES 32768          // 2 chunks (64 keys each) x [128 rows x 128 B]
-#define PF_V_STAGE 32768          // 2 chunks (64 dims each) x [128 keys x 128 B]
 #define PF_NONE (-FLT_MAX)        // reference maximum of a row no key of which has scored above -inf yet: finite, so that such scores are exponentials of -inf
 
 struct MlaPrefillArgs {

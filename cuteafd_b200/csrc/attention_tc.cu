@@ -55,7 +55,6 @@ struct AttnTcArgs {
   float scale;
 };
 
-__device__ __forceinline__ uint64_t desc_kmajor_sw128(uint32_t saddr) { return umma_desc_sw128(saddr); }
 // MN-major operand, 128-byte swizzle: 64-element MN blocks `lbo` bytes apart, 8-row K groups `sbo` bytes apart.
 __device__ __forceinline__ uint64_t desc_mnmajor_sw128(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
   uint64_t d = 0;

@@ -117,24 +117,20 @@ struct TcCfg {
   static_assert(KIND == KIND_BF16 ? ACC_COLS * NACC <= TMEM_COLS : ACC_COLS * NACC <= SFA_COL, "accumulators overlap the scale columns");
 };
 
-__device__ __forceinline__ uint32_t make_idesc(int kind, int n, uint32_t sf_id) {
+__device__ __forceinline__ uint32_t make_idesc(int kind, int n) {       // scale ids 0: `ti_mma4` sets those of its products
   uint32_t d = 0;
   if (kind == KIND_BF16) {
     d |= 1u << 4;            // fp32 accumulator
     d |= 1u << 7;            // A = bf16
     d |= 1u << 10;           // B = bf16
   } else if (kind == KIND_W4A8) {
-    d |= sf_id << 4;         // B scale-factor id: which byte of the 32-bit scale column this K = 32 step uses
     d |= 5u << 7;            // A = E2M1 (kind::mxf8f6f4 numbering: E4M3 0, E5M2 1, E2M3 3, E3M2 4, E2M1 5)
     d |= 0u << 10;           // B = E4M3
     d |= 1u << 23;           // UE8M0 scales
-    d |= sf_id << 29;        // A scale-factor id
   } else {
-    d |= sf_id << 4;         // B scale-factor id
     d |= 1u << 7;            // A = E2M1
     d |= 1u << 10;           // B = E2M1
     if (kind == KIND_MXFP4) d |= 1u << 23;   // UE8M0 scales (0 = UE4M3)
-    d |= sf_id << 29;        // A scale-factor id
   }
   d |= (uint32_t)(n >> 3) << 17;
   d |= (uint32_t)(128 >> 4) << 24;
@@ -315,7 +311,7 @@ __global__ void __launch_bounds__(192, TcCfg<KIND, TN, SWIGLU>::OCC) tc_linear_k
             for (int b = 0; b < C::NBLK; ++b) ti_cp_sf(tmem + C::SFB_COL + (4 * C::NBLK) * q + 4 * b, sfb + (b * C::SF_CHUNKS + q) * 32);
           }
         }
-        const uint32_t id = make_idesc(KIND, TN, 0), accum = kb > kb0 ? 1u : 0u;
+        const uint32_t id = make_idesc(KIND, TN), accum = kb > kb0 ? 1u : 0u;
         ti_mma4<C::ISSUE, 4, 4 * C::NBLK>(d0, dA, dB, id, accum, tmem + C::SFA_COL, tmem + C::SFB_COL);
         if (SWIGLU) ti_mma4<C::ISSUE, 4, 4 * C::NBLK>(d0 + TN, dA + C::A_BYTES / 16, dB, id, accum, tmem + C::SFA2_COL, tmem + C::SFB_COL);
         ti_commit(&empty_bar[s]);
@@ -744,7 +740,7 @@ __global__ void __launch_bounds__(192, 1) tc_linear_cluster_kernel(const __grid_
           ti_cp_sf(tmem + L::SFB_COL + 4 * q, sf0 + off + C::SFA_BYTES / 16 + q * 32);
         }
       }
-      ti_mma4<C::ISSUE, 4, 4>(tmem, dA, dA + C::A_BYTES / 16, make_idesc(KIND, TN, 0), kb > kb0 ? 1u : 0u, tmem + L::SFA_COL, tmem + L::SFB_COL);
+      ti_mma4<C::ISSUE, 4, 4>(tmem, dA, dA + C::A_BYTES / 16, make_idesc(KIND, TN), kb > kb0 ? 1u : 0u, tmem + L::SFA_COL, tmem + L::SFB_COL);
       ti_commit(&empty_bar[s]);
     }
     if (ok) ti_commit(&accf_bar);

@@ -9,6 +9,7 @@
 #pragma once
 #include "common.cuh"
 
+// K of a product: 16 (bf16), 64 (NVFP4, an E4M3 scale per 16; MXFP4, a UE8M0 scale per 32), 32 (E4M3; E2M1 x E4M3 with a UE8M0 scale per 32)
 enum { TI_F16 = 0, TI_NVF4 = 1, TI_MXF4 = 2, TI_F8 = 3, TI_W4A8 = 4 };
 
 #define TI_DESC_HI "0x40004040"        // upper word of an operand's descriptor: 1,024 bytes between groups of eight rows, 128-byte swizzle
@@ -56,7 +57,7 @@ __device__ __forceinline__ void ti_f16x4_ts(uint32_t d, uint32_t a_col, uint32_t
   asm volatile(TI_BEGIN TI_STEP_TS(0, "z") TI_STEP_TS(1, "t") TI_STEP_TS(2, "t") TI_STEP_TS(3, "t") "}"
                ::"r"(d), "r"(a_col), "r"(b_lo), "r"(accumulate), "r"(idesc), "n"(B_STEP) : "memory");
 }
-// 512 bytes of scales to four tensor-memory columns
+// 512 bytes of scales, 32 rows x 128 bits, to four tensor-memory columns, the same in all four lane quarters
 __device__ __forceinline__ void ti_cp_sf(uint32_t col, uint32_t s_lo) {
   asm volatile("{\n\t.reg .pred e;\n\t.reg .b64 s;\n\telect.sync _|e, 0xffffffff;\n\tmov.b64 s, {%1, " TI_SF_HI "};\n\t@e tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], s;\n\t}"
                ::"r"(col), "r"(s_lo) : "memory");
