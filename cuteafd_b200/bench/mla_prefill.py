@@ -82,11 +82,11 @@ def main():
         "gather_ctx": lambda: call("cuteafd_mla_gather_ctx", ptr(eng.kv[0]), ptr(md["page_table"]), ptr(eng._pf_starts), ptr(md["kv_len"]), ptr(eng._pf_lat), 1,
                                    a.context, md["page_table"].shape[1], eng.kv.shape[1], eng._pf_cap, st, stream()),
         "kv_b_expand_gemm": lambda: ops.tc_linear(w.ensure_kvb(), eng._pf_act, eng._pf_kvb, rows=rows, status=eng.status),
-        "mla_prefill_kernel": lambda: call("cuteafd_mla_prefill_attention", ptr(q_nope), ptr(b["q_rope"]), ptr(eng._pf_kvb), ptr(eng._pf_lat), eng._pf_cap,
+        "mla_prefill_attention": lambda: call("cuteafd_mla_prefill_attention", ptr(q_nope), ptr(b["q_rope"]), ptr(eng._pf_kvb), ptr(eng._pf_lat), eng._pf_cap,
                                            ptr(eng._pf_starts), ptr(md["kv_len"]), ptr(md["q_start"]), ptr(md["q_len"]), ptr(b["o_tok"]), a.chunk, 1,
                                            a.chunk, Hl, scale, st, stream()),
     }
-    flops = {"gather_ctx": 0.0, "kv_b_expand_gemm": 2.0 * rows * 512 * Hl * 256, "mla_prefill_kernel": 2.0 * keys_seen * Hl * (192 + 128)}
+    flops = {"gather_ctx": 0.0, "kv_b_expand_gemm": 2.0 * rows * 512 * Hl * 256, "mla_prefill_attention": 2.0 * keys_seen * Hl * (192 + 128)}
     peaks = {}
     path = os.path.join(os.path.dirname(os.path.dirname(os.path.dirname(os.path.abspath(__file__)))), "MEASURED_PEAKS.json")
     if os.path.exists(path):

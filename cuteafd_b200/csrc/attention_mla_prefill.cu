@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) mla_prefill_kernel(const __grid
 // head_in_group) and walks the sequence's pages two at a time (128-key tiles), K and V straight from the paged store.  Causal
 // mask, optional sliding window and sink logit as in the decode kernel (attention_tc.cu), no split-KV: a prefill chunk has
 // enough query tiles to fill the GPU.  window < 0 drops the causal mask (bidirectional attention of a vision / audio encoder:
-// every query row sees keys [0, kvlen)).  The 64-key decode kernel spends 8 + 4 tcgen05.mma per 64 keys; this one 8 + 8 per 128 keys.
+// every query row sees keys [0, kvlen)).  Which steps without a window take the kernel of attention_prefill_pair.cuh instead: `pf_tiles_paged`.  The 64-key decode kernel spends 8 + 4 tcgen05.mma per 64 keys; this one 8 + 8 per 128 keys.
 template <int KC, int VC>
 struct GqaPrefillCfg {
   static constexpr int K_STAGE = KC * 16384, V_STAGE = VC * 16384;          // chunks (64 dims each) x [128 keys x 128 B]

@@ -13,8 +13,8 @@
 // Key tiles, the reference maximum's rule and every sum are those of the one-tile kernels: all of a row's values are added key after key, so
 // both give the same bits.
 // Measured, one-tile kernel / this one: 4096 rows of 64 heads over 4: 643 / 285 us; 2048 rows over 8192 keys of 128 latent heads: 1432 / 1127
-// (a pair takes 3,700 and 4,200 cycles a key tile, 2,048 and 2,560 of them of the tensor pipe; what it waits for is the chain from the last part of P
-// to the next scores).
+// (a pair takes 3,650 and 4,250 cycles a key tile, 2,048 and 2,560 of them of the tensor pipe: each softmax 1,830, 440 of them the maximum, and its wait for the next scores
+// 1,700 and 2,400.  One tile alone takes 3,210, of which 1,375 are that wait: the chain from the last part of P through P V and the scores, which nothing hides within a tile).
 #pragma once
 #include "tc_issue.cuh"
 

@@ -16,8 +16,12 @@
 //   Of a K in parts every part is read and added to registers before the next one starts.
 //   FP8: two 256-column buffers; every 128 channels of K is one product of its own, which the epilogue warps add, times its two scales, to
 //   fp32 registers: one FMA per output and scale block, because a thread's row has one activation scale and its 128 columns one weight scale.
-// What bounds it: a stage of 48 KB (54 KB with FP4 scales) per 512 (bf16, FP8) or 256 cycles (FP4) of products is 94 or 211 bytes per cycle and SM, of which
-// L2 gives 60 to 70: FP8 runs at 0.6 of its peak, FP4 at 0.4.
+// What bounds it: the four products of a stage take 512 cycles whatever the kind, over 48 KB of operands (54 KB with FP4 scales).  Measured cycles a stage, and what the
+// issuer waits for in them:
+//   bf16, 4096 x 12288 x 2048                    686   operands 549 (the producer 326 for a free stage), accumulator 21
+//   NVFP4 / MXFP4, 4096 x 9216 x 4096            987 / 970   operands 531 / 469 (producer 123 / 117), then activation scales 192 / 147, accumulator 30
+//   FP8, 2048 x 7168 x 16384; 2048 x 24576 x 1536   754; 1169   accumulator 419; 761 (the epilogue's promotion), operands 153; 193
+// So FP4 waits for loads that are in flight, four stages of them (reads from L2 run at 38 % of their peak, in bf16 at 50 %), and FP8 for the epilogue.
 #define CA_PDL_CLASS 1
 #include "tc_gemm_wide.cuh"
 #include "tc_issue.cuh"

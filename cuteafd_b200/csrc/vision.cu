@@ -1,6 +1,6 @@
 // Pointwise kernels of the vision tower (a ViT encoder in front of the decoder: patch embedding, `depth` pre-norm blocks of
 // bidirectional multi-head attention + MLP, a 2x2 spatial merger).  The GEMMs are `tc_linear` (bf16 tcgen05), the attention is
-// `gqa_prefill_kernel` in its bidirectional mode over a scratch paged store whose heads are zero-padded to 128 dimensions; what is
+// `prefill_pair_kernel` in its bidirectional mode over a scratch paged store whose heads are zero-padded to 128 dimensions; what is
 // left is memory-bound glue, fused so that every activation crosses HBM once per block half:
 //   rgb_patches      resized RGB8 image -> normalised bf16 patch rows in merge-group order (the order the merger concatenates)
 //   add_norm         x (fp32 residual) += y + bias of the GEMM before, then LayerNorm / RMSNorm to the bf16 input of the next GEMM

@@ -381,7 +381,7 @@ class MlaEngine(Engine):
 
     def _prefill_attention(self, li: int, w, b: dict, sh: StepShape, q_nope: torch.Tensor):
         """gather the context's latent rows -> expand them to per-head keys / values (one GEMM with kv_b) -> per-head causal
-        attention (`mla_prefill_kernel`), output token-major in b["o_tok"].  Reference: glm_mla_prefill.cu:123-960."""
+        attention (`prefill_pair_kernel` or `mla_prefill_kernel`), output token-major in b["o_tok"].  Reference: glm_mla_prefill.cu:123-960."""
         a, Hl, dev = self.spec.attn, self.heads_local, self.device
         n_seq, md = sh.n_seq, self.md
         kv, rows = self._ctx_plan(sh)

@@ -1,7 +1,7 @@
 """Vision tower on the GPU: images -> rows of the decoder's hidden size that replace the image placeholder tokens of a prompt.
 
 The tower is a ViT encoder (`ref/vision.py` is its fp32 oracle and holds `VisionSpec`).  On the device every matrix product is a
-bf16 `tc_linear` (tcgen05), the attention is `gqa_prefill_kernel` in its bidirectional mode (window = -1) reading a scratch paged
+bf16 `tc_linear` (tcgen05), the attention is `prefill_pair_kernel` in its bidirectional mode (window = -1) reading a scratch paged
 store, with the heads zero-padded from `head_dim` to the kernel's 128 dimensions (zero key dimensions add nothing to a score, zero
 value dimensions come out as zero and meet zero columns of the padded output projection), and the glue is `csrc/vision.cu`: the
 residual stays fp32, every GEMM reads bf16 rows written by the fused add + norm / bias + activation kernels.  All images of a call
